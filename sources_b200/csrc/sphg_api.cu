@@ -18,6 +18,7 @@
 
 #include "../../include/sphg.h"
 #include "sphg_kernels.cuh"
+#include "sphg_kernels2.cuh"
 
 namespace {
 
@@ -914,6 +915,64 @@ struct Engine : EngineBase {
     // The pair passes of one step for kernel function SKF.  fh: run the
     // leapfrog predictor inside the gathers; u: what the last pass of each
     // phase does after its sums (nothing, or the corrector).
+    // FP32 with one h for all particles: two particles per lane pair in
+    // packed FP32 arithmetic (sphg_pairs2.cuh); else one particle per lane.
+    bool paired() const { return sizeof(T) == 4 && sc_same.uniform; }
+    // dspp: the wall force's r0
+    template <int SKF>
+    PairK pair_k(double dspp = 0.0) const {
+        const double h = (double)(float)hrange[0][1], pi = SPHG_PI_REF;
+        PairK K{};
+        K.h = (float)h;
+        K.nih = (float)(-1.0 / h);
+        K.ks = K.kw = 1.0f;
+        if (SKF == 1) {
+            const double fac = 15.0 / (7.0 * pi * h * h);
+            K.sn1 = (float)(3.0 / h); K.sn0 = (float)(4.0 / h);
+            K.ks = (float)(-fac / (2.0 * h)); K.kw = (float)(fac / 6.0);
+        } else if (SKF == 4) {
+            const double fac = 7.0 / (4.0 * pi * h * h);
+            K.ks = (float)(-5.0 * fac / (h * h)); K.kw = (float)fac;
+        }
+        const bool visc = sim.visc_artificial != 0;
+        K.nh = (float)-h;
+        K.h2e = (float)(sim.etq * sim.etq * h * h);
+        K.alpha = visc ? (float)(0.5 * sim.alpha) : 0.0f;
+        K.beta = visc ? (float)sim.beta : 0.0f;
+        K.alpha_c = (float)(2.0 * sim.s_c);
+        K.r0 = (float)dspp; K.dd = (float)(sim.dd / (double)K.ks); K.p1 = (float)sim.p1; K.p2 = (float)sim.p2;
+        K.kb = (float)sim.s_kb;
+        K.thr = sc_same.r2_uniform;
+        return K;
+    }
+    static int blocks2(int n) { return blocks(n, SPHG_TPB2); }
+    template <int SKF>
+    int launch_water_a(PhaseDev<T>& D) {
+        if constexpr (sizeof(T) == 4)
+            if (paired())
+                return launch_pdl("water_pass_a", k_water_pass_a2<SKF>, blocks2(D.n), SPHG_TPB2, Staged2<false>::BYTES, D, grid,
+                                  pair_k<SKF>(), sim, cnt);
+        return launch_pdl("water_pass_a", k_water_pass_a<T, SKF, false>, blocks(D.n, SPHG_TPB), SPHG_TPB,
+                          (size_t)SPHG_STAGE_A * (16 + sizeof(RecA<T>)), D, grid, sc_same, sim, cnt);
+    }
+    template <int SKF, bool FCH>
+    int launch_water_b(PhaseDev<T>& D, PhaseDev<T>& O, const StepCtl& u) {
+        if constexpr (sizeof(T) == 4)
+            if (paired())
+                return launch_pdl("water_pass_b", k_water_pass_b2<SKF, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O,
+                                  grid, pair_k<SKF>(D.dspp), sim, u, cnt);
+        return launch_pdl("water_pass_b", k_water_pass_b<T, SKF, false, FCH>, blocks(D.n, SPHG_TPB), SPHG_TPB, 0, D, O, grid,
+                          sc_same, sc_cross, sim, u, cnt);
+    }
+    template <int SKF, bool SINGLE, bool FCH>
+    int launch_soil(PhaseDev<T>& D, PhaseDev<T>& O, int slot, const StepCtl& u) {
+        if constexpr (sizeof(T) == 4)
+            if (paired())
+                return launch_pdl("soil_pass", k_soil_pass2<SKF, SINGLE, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O, grid,
+                                  pair_k<SKF>(D.dspp), sim, cnt, slot, u);
+        return launch_pdl("soil_pass", k_soil_pass<T, SKF, SINGLE, FCH>, blocks(D.n, SPHG_TPB), SPHG_TPB, 0, D, O, grid, sc_same,
+                          sc_cross, sim, cnt, slot, u);
+    }
     template <int SKF>
     int passes(int fh, StepCtl u) {
         const sphg_params& p = ctx->prm;
@@ -935,8 +994,7 @@ struct Engine : EngineBase {
                 if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 1, dp, fh, 0, dp, cnt))) return rc;
                 StepCtl us = u; us.with_vof = 0; us.do_dp = dp;
                 us.ncount = u.update ? counts[0] : nullptr;
-                if ((rc = launch_pdl("soil_pass", k_soil_pass<T, SKF, true, false>, blocks(D.n, tpb), tpb, 0, D, D, grid, sc_same, sc_same,
-                                 sim, cnt, 0, us))) return rc;
+                if ((rc = launch_soil<SKF, true, false>(D, D, 0, us))) return rc;
             }
         } else {
             PhaseDev<T>& W = P[0];
@@ -947,9 +1005,7 @@ struct Engine : EngineBase {
             us.ncount = u.update ? counts[1] : nullptr;
             // the soil's gather was launched by run() on the side stream
             if ((rc = launch_pdl("gather", k_gather<T>, blocks(W.n, 256), 256, 0, W, sim, 0, 0, fh, 1, 0, cnt))) return rc;
-            if ((rc = launch_pdl("water_pass_a", k_water_pass_a<T, SKF, false>, blocks(W.n, tpb), tpb,
-                                  (size_t)SPHG_STAGE_A * (16 + sizeof(RecA<T>)), W, grid, sc_same, sim, cnt)))
-                return rc;
+            if ((rc = launch_water_a<SKF>(W))) return rc;
             // The cross pairs run inside the last pass of each phase; the soil
             // pass reads the water pressure that water_pass_a sets.  After
             // water_pass_a the two last passes share no data: each reads the
@@ -967,10 +1023,7 @@ struct Engine : EngineBase {
                 CUDA_TRY(cudaStreamWaitEvent(side, ctx->ev_fork, 0));
             }
             ctx->stream = side;
-            rc = fch ? launch_pdl("soil_pass", k_soil_pass<T, SKF, false, true>, blocks(S.n, tpb), tpb, 0, S, W, grid, sc_same,
-                              sc_cross, sim, cnt, 1, us)
-                     : launch_pdl("soil_pass", k_soil_pass<T, SKF, false, false>, blocks(S.n, tpb), tpb, 0, S, W, grid, sc_same,
-                              sc_cross, sim, cnt, 1, us);
+            rc = fch ? launch_soil<SKF, false, true>(S, W, 1, us) : launch_soil<SKF, false, false>(S, W, 1, us);
             cudaError_t ej = side != main_stream ? cudaEventRecord(ctx->ev_join, side) : cudaSuccess;
             ctx->stream = main_stream;
             // water_pass_b reads the soil's records: wait for the soil's gather
@@ -979,10 +1032,7 @@ struct Engine : EngineBase {
                 if (e2 != cudaSuccess && rc == 0) rc = SPHG_ERR_CUDA;
             }
             if (rc == 0)
-                rc = fch ? launch_pdl("water_pass_b", k_water_pass_b<T, SKF, false, true>, blocks(W.n, tpb), tpb, 0, W, S, grid,
-                                  sc_same, sc_cross, sim, uw, cnt)
-                         : launch_pdl("water_pass_b", k_water_pass_b<T, SKF, false, false>, blocks(W.n, tpb), tpb, 0, W, S, grid,
-                                  sc_same, sc_cross, sim, uw, cnt);
+                rc = fch ? launch_water_b<SKF, true>(W, S, uw) : launch_water_b<SKF, false>(W, S, uw);
             // join in every case, so that a capture in progress ends joined
             cudaError_t ew = ej != cudaSuccess ? ej
                              : side != main_stream ? cudaStreamWaitEvent(main_stream, ctx->ev_join, 0) : cudaSuccess;

@@ -331,6 +331,19 @@ __device__ __forceinline__ void pair_kernel(const KernelConst<T, SKF>& ka, const
 // sum_density (m_particles.f90:2243-2298) and the df2 divergence of the
 // water-only step, drho = -rho*(df2(vx,'x') + df2(vy,'y'))
 // (declarations_sph.f90:1465-1466, df2 m_particles.f90:1802-1831).
+template <typename T>
+__device__ __forceinline__ void water_sum_finish(const PhaseDev<T>& P, int k, const RecA<T>& ra, T num, T wi, T sx, T sy,
+                                                 int hits) {
+    const int a = P.perm[k];
+    const T rho = num / wi;
+    P.rho[a] = (double)rho;
+    P.drho[a] = -rho * (sx / rho + sy / rho);
+    RecA<T> r2;
+    r2.vx = ra.vx; r2.vy = ra.vy; r2.vol = (T)(P.mass[a] / (double)rho); r2.rho = rho;
+    P.recA2[k] = r2;
+    P.countiac[a] = hits;
+}
+
 template <typename T, int SKF>
 __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom g, SearchConst sc, SimConst c, DevCounters* cnt) {
     pdl_enter();
@@ -362,17 +375,52 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
         sy += mb * ((rb.vy - ra.vy) * (sr * dy));
     });
     if (valid) {
-        const int a = P.perm[k];
-        const T rho = num / wi;
-        P.rho[a] = (double)rho;
-        P.drho[a] = -rho * (sx / rho + sy / rho);
-        RecA<T> r2;
-        r2.vx = ra.vx; r2.vy = ra.vy; r2.vol = (T)(P.mass[a] / (double)rho); r2.rho = rho;
-        P.recA2[k] = r2;
-        P.countiac[a] = hits;
         if (P.hmask) P.hmask[k] = mask;
+        water_sum_finish(P, k, ra, num, wi, sx, sy, hits);
     }
     count_stats(cnt, 0, 0, hits, valid);
+}
+
+// What water_pass_a does with a particle's sums: EOS, newtonian_fluid, the
+// record of the next pass, the interaction count.
+template <typename T, bool SINGLE>
+__device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimConst& c, int k, T con, T dl, T t0, T t1, T t2,
+                                               T t3, int hits) {
+    const T c23 = (T)SPHG_F32LIT(2.0f / 3.0f);
+    const int a = P.perm[k];
+    T txx, txy, tyy, drho;
+    double p, cnew, vof;
+    const double rho = P.rho[a];
+    if (SINGLE) {
+        drho = P.drho[a] + dl;
+        txx = c23 * (T(2) * t0 - t1);
+        txy = t2 + t3;
+        tyy = c23 * (T(2) * t1 - t0);
+        p = P.p[a];
+        if (rho > 0.0) p = c.tab[P.sid[a]].w_b * (pow(rho / c.w_rho0, c.w_gamma) - 1);
+        cnew = P.c[a];
+        vof = 1.0;
+    } else {
+        drho = con + dl;
+        txx = t0; txy = t1; tyy = t2;
+        vof = P.vof[a];
+        const double ratio = rho / (c.w_rho0 * vof);
+        const SceneTab& st = c.tab[P.sid[a]];
+        p = st.w_b * (pow(ratio, c.w_gamma) - 1);
+        cnew = st.w_c * pow(ratio, 3.0);
+        P.c[a] = cnew;
+    }
+    P.drho[a] = drho;
+    P.p[a] = p;
+    // newtonian_fluid: sxx = mu*txx in place (sxx and txx are one array)
+    const double sxx = c.w_mu * (double)txx, sxy = c.w_mu * (double)txy, syy = c.w_mu * (double)tyy;
+    P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy;
+    RecB<T> rb;
+    rb.p = (T)p; rb.c = (T)cnew; rb.vof = (T)vof;
+    rb.sxx = (T)sxx; rb.sxy = (T)sxy; rb.syy = (T)syy;
+    rb.itype = (T)P.itype[a]; rb.aux = T(0);
+    P.recB[k] = rb;
+    if (!SINGLE) P.countiac[a] = hits;
 }
 
 // ----------------------------------------------------------- water: pass A
@@ -452,40 +500,8 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : 1) k_
         }
     }
     if (valid) {
-        T txx, txy, tyy, drho;
-        double p, cnew, vof;
-        const double rho = P.rho[a];
-        if (SINGLE) {
-            drho = P.drho[a] + dl;
-            txx = c23 * (T(2) * t0 - t1);
-            txy = t2 + t3;
-            tyy = c23 * (T(2) * t1 - t0);
-            p = P.p[a];
-            if (rho > 0.0) p = c.tab[P.sid[a]].w_b * (pow(rho / c.w_rho0, c.w_gamma) - 1);
-            cnew = P.c[a];
-            vof = 1.0;
-        } else {
-            drho = con + dl;
-            txx = t0; txy = t1; tyy = t2;
-            vof = P.vof[a];
-            const double ratio = rho / (c.w_rho0 * vof);
-            const SceneTab& st = c.tab[P.sid[a]];
-            p = st.w_b * (pow(ratio, c.w_gamma) - 1);
-            cnew = st.w_c * pow(ratio, 3.0);
-            P.c[a] = cnew;
-        }
-        P.drho[a] = drho;
-        P.p[a] = p;
-        // newtonian_fluid: sxx = mu*txx in place (sxx and txx are one array)
-        const double sxx = c.w_mu * (double)txx, sxy = c.w_mu * (double)txy, syy = c.w_mu * (double)tyy;
-        P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy;
-        RecB<T> rb;
-        rb.p = (T)p; rb.c = (T)cnew; rb.vof = (T)vof;
-        rb.sxx = (T)sxx; rb.sxy = (T)sxy; rb.syy = (T)syy;
-        rb.itype = (T)P.itype[a]; rb.aux = T(0);
-        P.recB[k] = rb;
-        P.countiac[a] = hits;
         if (!SINGLE) P.hmask[k] = mask;
+        water_a_finish<T, SINGLE>(P, c, k, con, dl, t0, t1, t2, t3, hits);
     }
     if (!SINGLE) count_stats(cnt, 0, 0, hits, valid);
 }
@@ -544,6 +560,60 @@ __device__ __forceinline__ int cross_water_sums(HB& hb, const PhaseDev<T>& S, co
         dvof -= mb * (sr * (ux * dx + uy * dy));
         v2 += mb * w;
     });
+}
+
+// A water particle's sums of water_pass_b: momentum (before the division by
+// rho), artificial viscosity plus wall force, XSPH, delta-SPH on vof, and the
+// cross pairs' sums.
+template <typename T>
+struct WaterB {
+    T mx, my, fx, fy, xsx, xsy, dvf;
+    T cdx, cdy, cdvof, cv2;
+    int chits;
+};
+
+// What water_pass_b does with them: the rates, the renormalisation, the
+// leapfrog corrector and the next step's cell key.
+template <typename T, bool SINGLE>
+__device__ __forceinline__ void water_b_finish(const PhaseDev<T>& P, const GridGeom& g, const SimConst& c, const StepCtl& u,
+                                               DevCounters* cnt, int k, T rho_a, T phia, const WaterB<T>& w) {
+    typedef typename V2<T>::t T2;
+    const int a = P.perm[k];
+    T dvx = w.mx, dvy = w.my;
+    if (rho_a > T(0)) { dvx = dvx / rho_a; dvy = dvy / rho_a; }
+    dvx = dvx + w.fx;
+    dvy = dvy + w.fy + (T)c.gravity;
+    if (c.average_velocity) {
+        const bool real_a = P.itype[a] > 0;
+        const T eps = (T)c.epsilon;
+        T2 av; av.x = real_a ? eps * w.xsx : w.xsx; av.y = real_a ? eps * w.xsy : w.xsy;
+        P.av[a] = av;
+    }
+    if constexpr (SINGLE) {
+        T2 o; o.x = dvx; o.y = dvy;
+        P.dv[a] = o;
+        if (u.update) update_one(P, a, c, u.first, 0, 0);   // last pass of the water-only step
+    } else {
+        const T fd = phia * (T)(-c.numeric_gravity / c.s_perm);
+        T2 o; o.x = dvx + fd * w.cdx; o.y = dvy + fd * w.cdy;
+        P.dv[a] = o;
+        if (c.volume_fraction) {
+            const T irho0 = (T)(1.0 / c.s_rho0);
+            P.dvof[a] = w.dvf + w.cdvof * irho0;
+            const T vof2 = T(1) - w.cv2 * irho0;
+            P.vof2[a] = vof2;
+            if (c.renorm_now) {
+                double rho = P.rho[a] / P.vof[a];
+                P.vof[a] = (double)vof2;
+                P.rho[a] = rho * (double)vof2;
+            }
+        } else {
+            P.dvof[a] = w.dvf;
+        }
+        P.countiac[a] = w.chits;
+        if (u.update) update_one(P, a, c, u.first, u.with_vof, 0);   // last pass of the water phase
+    }
+    if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
 }
 
 // ----------------------------------------------------------- water: pass B
@@ -647,49 +717,102 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : 1) k_
                     [&](int m, T dx, T dy) { body(rec, P.recB, m, dx, dy); });
     const T d1x = d1.x, d1y = d1.y, d2x = d2.x, d2y = d2.y, d3x = d3.x, d3y = d3.y;
     const T avx = av.x, avy = av.y, rpx = rp.x, rpy = rp.y, xsx = xv.x, xsy = xv.y;
-    T dvx = -(phia * d1x) + d2x + d3x;
-    T dvy = -(phia * d1y) + d2y + d3y;
-    if (ra.rho > T(0)) { dvx = dvx / ra.rho; dvy = dvy / ra.rho; }
-    dvx = dvx + avx + rpx;
-    dvy = dvy + avy + rpy + (T)c.gravity;
-    if (valid && xsph) {
+    WaterB<T> w;
+    w.mx = -(phia * d1x) + d2x + d3x;
+    w.my = -(phia * d1y) + d2y + d3y;
+    w.fx = avx + rpx; w.fy = avy + rpy;
+    w.xsx = xsx; w.xsy = xsy;
+    w.dvf = dvf;
+    w.cdx = w.cdy = w.cdvof = w.cv2 = T(0);
+    w.chits = 0;
+    if constexpr (!SINGLE)
+        w.chits = cross_water_sums<T, SKF, FCH>(hb, S, g, scx, c, ka, xa, ha, ra, valid, w.cdx, w.cdy, w.cdvof, w.cv2);
+    if (valid) water_b_finish<T, SINGLE>(P, g, c, u, cnt, k, ra.rho, phia, w);
+    if constexpr (!SINGLE) count_stats(cnt, 2, -1, w.chits, valid);
+}
+
+// A soil particle's sums of soil_pass: momentum (before the division by rho),
+// artificial viscosity plus wall force, XSPH, the rates, and the cross pairs'
+// sums.
+template <typename T>
+struct SoilSums {
+    T mx, my, fx, fy, xsx, xsy;
+    T drho, txx, txy, tyy, vcc, wxy, dp, dsx, dsxy, dsy;
+    T cdx, cdy, cpx, cpy;
+    int hits;
+};
+
+// What soil_pass does with them: plastic_or_not, plastic_flow_rule3 and
+// Jaumann_rate on the post-DP state, the rates, the leapfrog corrector and
+// the next step's cell key.
+template <typename T, bool SINGLE>
+__device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom& g, const SimConst& c, const StepCtl& u,
+                                            DevCounters* cnt, int k, T rho_a, T phis, const SoilSums<T>& w, int& fail,
+                                            int& fail3) {
+    typedef typename V2<T>::t T2;
+    const int a = P.perm[k];
+    T dvx = w.mx, dvy = w.my;
+    if (rho_a > T(0)) { dvx = dvx / rho_a; dvy = dvy / rho_a; }
+    dvx = dvx + w.fx;
+    dvy = dvy + w.fy + (T)c.gravity;
+    if (c.average_velocity) {
+        const bool real_a = P.itype[a] > 0;
         const T eps = (T)c.epsilon;
-        T2 av; av.x = real_a ? eps * xsx : xsx; av.y = real_a ? eps * xsy : xsy;
+        T2 av; av.x = real_a ? eps * w.xsx : w.xsx; av.y = real_a ? eps * w.xsy : w.xsy;
         P.av[a] = av;
     }
-    if constexpr (SINGLE) {
-        if (valid) {
-            T2 o; o.x = dvx; o.y = dvy;
-            P.dv[a] = o;
-            if (u.update) update_one(P, a, c, u.first, 0, 0);   // last pass of the water-only step
-            if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
-        }
-    } else {
-        T cdx = 0, cdy = 0, cdvof = 0, cv2 = 0;
-        const int chits = cross_water_sums<T, SKF, FCH>(hb, S, g, scx, c, ka, xa, ha, ra, valid, cdx, cdy, cdvof, cv2);
-        if (valid) {
-            const T fd = phia * (T)(-c.numeric_gravity / c.s_perm);
-            T2 o; o.x = dvx + fd * cdx; o.y = dvy + fd * cdy;
-            P.dv[a] = o;
-            if (c.volume_fraction) {
-                const T irho0 = (T)(1.0 / c.s_rho0);
-                P.dvof[a] = dvf + cdvof * irho0;
-                const T vof2 = T(1) - cv2 * irho0;
-                P.vof2[a] = vof2;
-                if (c.renorm_now) {
-                    double rho = P.rho[a] / P.vof[a];
-                    P.vof[a] = (double)vof2;
-                    P.rho[a] = rho * (double)vof2;
-                }
-            } else {
-                P.dvof[a] = dvf;
+    P.drho[a] = w.drho;
+    // plastic_or_not + plastic_flow_rule3 + Jaumann_rate on the post-DP state
+    const double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
+    const double dtxx = (double)w.txx, dtxy = (double)w.txy, dtyy = (double)w.tyy, dvcc = (double)w.vcc;
+    const double G = c.s_E / (2.0 * (1 + c.s_niu));
+    double ds0 = 0.0, ds1 = 0.0, ds2 = 0.0, dp = 0.0;
+    fail = 0;
+    if (c.plasticity == 3) {
+        const double J2a = sqrt((sxx * sxx + 2.0 * (sxy * sxy) + syy * syy + (sxx + syy) * (sxx + syy)) / 2.0) + 1.0e-6;
+        const double alpha1 = c.tab[P.sid[a]].s_alpha1;
+        if (fabs(J2a - alpha1 * (3.0 * p)) < SPHG_F32LIT(1.0e-5f)) fail = 1;
+        P.fail[a] = fail;
+        if (fail) {
+            const double exx = dtxx / 2.0 + dvcc / 3.0, exy = dtxy / 2.0, eyy = dtyy / 2.0 + dvcc / 3.0;
+            const double sde = sxx * exx + 2.0 * sxy * exy + syy * eyy;
+            double J2 = (sxx * sxx + 2.0 * (sxy * sxy) + syy * syy + (sxx + syy) * (sxx + syy)) / 2.0;
+            J2 = J2 + 1.0e-10;
+            const double al = alpha1, K = c.s_k;
+            const double dlambda = (3.0 * al * K * dvcc + G / sqrt(J2) * sde) / (9.0 * (al * al) * K + G);
+            if (!(dlambda < 0)) {
+                ds0 = ds0 - dlambda * (G / sqrt(J2) * sxx);
+                ds1 = ds1 - dlambda * (G / sqrt(J2) * sxy);
+                ds2 = ds2 - dlambda * (G / sqrt(J2) * syy);
+                dp = dp + 3.0 * K * al * dlambda;
+                P.eps_p[a] = P.eps_p[a] + dlambda * sxy / (2 * sqrt(J2)) * SPHG_F32LIT(0.000005f);
             }
-            P.countiac[a] = chits;
-            if (u.update) update_one(P, a, c, u.first, u.with_vof, 0);   // last pass of the water phase
-            if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
         }
-        count_stats(cnt, 2, -1, chits, valid);
     }
+    const double dwxy = (double)w.wxy;
+    ds0 = ds0 + G * dtxx; ds1 = ds1 + G * dtxy; ds2 = ds2 + G * dtyy;
+    dp = dp - c.s_k * dvcc;
+    ds0 = ds0 + 2.0 * sxy * dwxy;
+    ds1 = ds1 - (sxx - syy) * dwxy;
+    ds2 = ds2 - 2.0 * sxy * dwxy;
+    P.dsxx[a] = (T)(ds0 + (double)w.dsx);
+    P.dsxy[a] = (T)(ds1 + (double)w.dsxy);
+    P.dsyy[a] = (T)(ds2 + (double)w.dsy);
+    P.dp[a] = (T)(dp + (double)w.dp);
+    P.c[a] = c.s_c;
+    P.txx[a] = w.txx; P.tyy[a] = w.tyy; P.txy[a] = w.wxy;   // wxy is txy (alias)
+    P.vcc[a] = w.vcc;
+    P.countiac[a] = w.hits;
+    T2 o; o.x = dvx; o.y = dvy;
+    if constexpr (!SINGLE) {
+        const T irs = T(1) / rho_a;
+        const T fd = phis * (T)(-c.numeric_gravity / c.s_perm) * irs, fp = irs * phis;
+        o.x = dvx + (fd * w.cdx + fp * w.cpx); o.y = dvy + (fd * w.cdy + fp * w.cpy);
+        if (c.volume_fraction) P.vof[a] = P.rho[a] / c.s_rho0;
+    }
+    P.dv[a] = o;
+    fail3 = u.update ? update_one(P, a, c, u.first, SINGLE ? 0 : u.with_vof, u.do_dp) : 0;   // last pass of the soil phase
+    if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
 }
 
 // ------------------------------------------------------------------ soil
@@ -804,81 +927,23 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : 1)
             xsy += q * dv;
         }
     });
-    int fail = 0, fail3 = 0;
-    T dvx, dvy;
-    if (SINGLE) { dvx = -s1x + s2x + s3x; dvy = -s1y + s2y + s3y; }
+    SoilSums<T> w;
+    if (SINGLE) { w.mx = -s1x + s2x + s3x; w.my = -s1y + s2y + s3y; }
     else {
-        dvx = -(s1x * ra.rho) + s2x * ra.rho + s3x * ra.rho;
-        dvy = -(s1y * ra.rho) + s2y * ra.rho + s3y * ra.rho;
+        w.mx = -(s1x * ra.rho) + s2x * ra.rho + s3x * ra.rho;
+        w.my = -(s1y * ra.rho) + s2y * ra.rho + s3y * ra.rho;
     }
-    if (ra.rho > T(0)) { dvx = dvx / ra.rho; dvy = dvy / ra.rho; }
-    dvx = dvx + avx + rpx;
-    dvy = dvy + avy + rpy + (T)c.gravity;
-    if (valid) {
-        if (SINGLE) { T2 o; o.x = dvx; o.y = dvy; P.dv[a] = o; }
-        if (xsph) {
-            const T eps = (T)c.epsilon;
-            T2 av; av.x = real_a ? eps * xsx : xsx; av.y = real_a ? eps * xsy : xsy;
-            P.av[a] = av;
-        }
-        P.drho[a] = con + dl;
-        // plastic_or_not + plastic_flow_rule3 + Jaumann_rate on the post-DP state
-        const double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
-        const double dtxx = (double)txx, dtxy = (double)txy, dtyy = (double)tyy, dvcc = (double)vcc;
-        const double G = c.s_E / (2.0 * (1 + c.s_niu));
-        double ds0 = 0.0, ds1 = 0.0, ds2 = 0.0, dp = 0.0;
-        if (c.plasticity == 3) {
-            const double J2a = sqrt((sxx * sxx + 2.0 * (sxy * sxy) + syy * syy + (sxx + syy) * (sxx + syy)) / 2.0) + 1.0e-6;
-            const double alpha1 = c.tab[P.sid[a]].s_alpha1;
-            if (fabs(J2a - alpha1 * (3.0 * p)) < SPHG_F32LIT(1.0e-5f)) fail = 1;
-            P.fail[a] = fail;
-            if (fail) {
-                const double exx = dtxx / 2.0 + dvcc / 3.0, exy = dtxy / 2.0, eyy = dtyy / 2.0 + dvcc / 3.0;
-                const double sde = sxx * exx + 2.0 * sxy * exy + syy * eyy;
-                double J2 = (sxx * sxx + 2.0 * (sxy * sxy) + syy * syy + (sxx + syy) * (sxx + syy)) / 2.0;
-                J2 = J2 + 1.0e-10;
-                const double al = alpha1, K = c.s_k;
-                const double dlambda = (3.0 * al * K * dvcc + G / sqrt(J2) * sde) / (9.0 * (al * al) * K + G);
-                if (!(dlambda < 0)) {
-                    ds0 = ds0 - dlambda * (G / sqrt(J2) * sxx);
-                    ds1 = ds1 - dlambda * (G / sqrt(J2) * sxy);
-                    ds2 = ds2 - dlambda * (G / sqrt(J2) * syy);
-                    dp = dp + 3.0 * K * al * dlambda;
-                    P.eps_p[a] = P.eps_p[a] + dlambda * sxy / (2 * sqrt(J2)) * SPHG_F32LIT(0.000005f);
-                }
-            }
-        }
-        const double dwxy = (double)wxy;
-        ds0 = ds0 + G * dtxx; ds1 = ds1 + G * dtxy; ds2 = ds2 + G * dtyy;
-        dp = dp - c.s_k * dvcc;
-        ds0 = ds0 + 2.0 * sxy * dwxy;
-        ds1 = ds1 - (sxx - syy) * dwxy;
-        ds2 = ds2 - 2.0 * sxy * dwxy;
-        P.dsxx[a] = (T)(ds0 + (double)dsx);
-        P.dsxy[a] = (T)(ds1 + (double)dsxy);
-        P.dsyy[a] = (T)(ds2 + (double)dsy);
-        P.dp[a] = (T)(dp + (double)dpp);
-        P.c[a] = c.s_c;
-        P.txx[a] = txx; P.tyy[a] = tyy; P.txy[a] = wxy;   // wxy is txy (alias)
-        P.vcc[a] = vcc;
-        P.countiac[a] = hits;
-        if (SINGLE && u.update) fail3 = update_one(P, a, c, u.first, 0, u.do_dp);   // last pass of the soil-only step
-        if (SINGLE && u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
-    }
-    if constexpr (!SINGLE) {
-        T cdx = 0, cdy = 0, cpx = 0, cpy = 0;
-        cross_soil_sums<T, SKF, FCH>(hb, W, g, scx, c, ka, xa, ha, ra, valid, cdx, cdy, cpx, cpy);
-        if (valid) {
-            const T phis = qa.vof;
-            const T irs = T(1) / ra.rho;
-            const T fd = phis * (T)(-c.numeric_gravity / c.s_perm) * irs, fp = irs * phis;
-            T2 o; o.x = dvx + (fd * cdx + fp * cpx); o.y = dvy + (fd * cdy + fp * cpy);
-            P.dv[a] = o;
-            if (c.volume_fraction) P.vof[a] = P.rho[a] / c.s_rho0;
-            if (u.update) fail3 = update_one(P, a, c, u.first, u.with_vof, u.do_dp);   // last pass of the soil phase
-            if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
-        }
-    }
+    w.fx = avx + rpx; w.fy = avy + rpy;
+    w.xsx = xsx; w.xsy = xsy;
+    w.drho = con + dl;
+    w.txx = txx; w.txy = txy; w.tyy = tyy; w.vcc = vcc; w.wxy = wxy;
+    w.dp = dpp; w.dsx = dsx; w.dsxy = dsxy; w.dsy = dsy;
+    w.cdx = w.cdy = w.cpx = w.cpy = T(0);
+    w.hits = hits;
+    if constexpr (!SINGLE)
+        cross_soil_sums<T, SKF, FCH>(hb, W, g, scx, c, ka, xa, ha, ra, valid, w.cdx, w.cdy, w.cpx, w.cpy);
+    int fail = 0, fail3 = 0;
+    if (valid) soil_finish<T, SINGLE>(P, g, c, u, cnt, k, ra.rho, qa.vof, w, fail, fail3);
     count_stats(cnt, slot, slot, hits, valid);
     if (c.plasticity == 3) count_fail(cnt, 2, fail);
     if (u.update && u.do_dp) count_fail(cnt, 3, fail3);
