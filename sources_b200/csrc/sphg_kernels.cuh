@@ -192,49 +192,62 @@ __device__ __forceinline__ int first_half_one(const PhaseDev<T>& P, int a, const
     return fail;
 }
 
-// first_step (:686-723) when first != 0, else second_half (:725-762), plus the
-// Drucker-Prager call after it on soil (:583, :601, :1069, :1107).
+// The corrector: first_step (:686-723) when first != 0, else second_half
+// (:725-762), plus the Drucker-Prager call after it on soil (:583, :601,
+// :1069, :1107).  load() reads all of the particle's state it needs before any
+// result of the pass is stored (the stores could alias the loads, so reading
+// field by field between them made each load wait for the one before: the
+// last passes spent half their time so); apply() integrates and stores.
 template <typename T>
-__device__ __forceinline__ int update_one(const PhaseDev<T>& P, int a, const SimConst& c, int first, int with_vof, int do_dp) {
-    const SceneTab& st = c.tab[P.sid[a]];
-    const double dt = st.dt;
-    int fail = 0;
-    if (!c.summation_density)
-        P.rho[a] = first ? P.rho[a] + (dt / 2.0) * (double)P.drho[a] : P.rho_min[a] + dt * (double)P.drho[a];
-    if (with_vof && P.material == 1 && c.volume_fraction)
-        P.vof[a] = first ? P.vof[a] + (dt / 2.0) * (double)P.dvof[a] : P.vof_min[a] + dt * (double)P.dvof[a];
-    if (P.material == 2) {
-        double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
-        const double d0 = P.dsxx[a], d1 = P.dsxy[a], d2 = P.dsyy[a], d3 = P.dp[a];
-        if (c.stress_integration == 1) {
-            sxx = sxx + dt * d0; sxy = sxy + dt * d1; syy = syy + dt * d2; p = p + dt * d3;
-        } else if (c.stress_integration == 2) {
-            if (first) {
-                sxx = sxx + (dt / 2.0) * d0; sxy = sxy + (dt / 2.0) * d1;
-                syy = syy + (dt / 2.0) * d2; p = p + (dt / 2.0) * d3;
-            } else {
-                sxx = P.sxx_min[a] + dt * d0; sxy = P.sxy_min[a] + dt * d1;
-                syy = P.syy_min[a] + dt * d2; p = P.p_min[a] + dt * d3;
-            }
+struct Corrector {
+    typedef typename V2<T>::t T2;
+    double dt, rho, vof, alpha1, p, sxx, sxy, syy;
+    double2 v, x;
+    T drho;
+    bool real;
+    __device__ __forceinline__ void load(const PhaseDev<T>& P, int a, const SimConst& c, const StepCtl& u, bool soil) {
+        const int sid = P.sid[a];
+        real = P.itype[a] >= 0;
+        x = P.x[a];
+        v = u.first ? P.v[a] : P.v_min[a];
+        rho = u.first ? P.rho[a] : P.rho_min[a];
+        if (!soil) {
+            drho = P.drho[a];
+            vof = u.first ? P.vof[a] : P.vof_min[a];
+        } else if (c.stress_integration == 2 && !u.first) {
+            p = P.p_min[a]; sxx = P.sxx_min[a]; sxy = P.sxy_min[a]; syy = P.syy_min[a];
+        } else {
+            p = P.p[a]; sxx = P.sxx[a]; sxy = P.sxy[a]; syy = P.syy[a];
         }
-        if (do_dp) { fail = dp_return(p, sxx, sxy, syy, st.s_alpha1); P.fail[a] = fail; }
-        P.p[a] = p; P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy;
+        dt = c.tab[sid].dt;
+        alpha1 = soil ? c.tab[sid].s_alpha1 : 0.0;
     }
-    if (P.itype[a] >= 0) {
-        double2 v = first ? P.v[a] : P.v_min[a];
-        const typename V2<T>::t d = P.dv[a];
-        const typename V2<T>::t av = P.av[a];
-        double2 x = P.x[a];
+    // rho and v, x; the new position
+    __device__ __forceinline__ void move(const PhaseDev<T>& P, int a, const SimConst& c, int first, T2 d, T2 av) {
         const double h = first ? dt / 2.0 : dt;
-        v.x = v.x + h * (double)d.x + (double)av.x;
-        x.x = x.x + dt * v.x;
-        v.y = v.y + h * (double)d.y + (double)av.y;
-        x.y = x.y + dt * v.y;
-        P.v[a] = v;
-        P.x[a] = x;
+        if (!c.summation_density) P.rho[a] = rho + h * (double)drho;
+        if (real) {
+            v.x = v.x + h * (double)d.x + (double)av.x;
+            x.x = x.x + dt * v.x;
+            v.y = v.y + h * (double)d.y + (double)av.y;
+            x.y = x.y + dt * v.y;
+            P.v[a] = v;
+            P.x[a] = x;
+        }
     }
-    return fail;
-}
+    __device__ __forceinline__ int stress(const PhaseDev<T>& P, int a, const SimConst& c, int first, int do_dp, T dsxx, T dsxy,
+                                          T dsyy, T dp) {
+        const double h = c.stress_integration == 1 ? dt : first ? dt / 2.0 : dt;
+        sxx = sxx + h * (double)dsxx;
+        sxy = sxy + h * (double)dsxy;
+        syy = syy + h * (double)dsyy;
+        p = p + h * (double)dp;
+        int fail = 0;
+        if (do_dp) { fail = dp_return(p, sxx, sxy, syy, alpha1); P.fail[a] = fail; }
+        P.p[a] = p; P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy;
+        return fail;
+    }
+};
 
 __device__ __forceinline__ void count_fail(DevCounters* cnt, int slot, int fail) {
     int s = __syncthreads_count(fail);
@@ -381,6 +394,26 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
     count_stats(cnt, 0, 0, hits, valid);
 }
 
+// r^3 to within rounding: the product and the rounding errors of its factors.
+__device__ __forceinline__ double cube(double r) {
+    const double r2 = r * r, e2 = fma(r, r, -r2), r3 = r2 * r;
+    return r3 + (fma(r2, r, -r3) + e2 * r);
+}
+// r^gamma - 1 of the Tait equation.  gamma = 7, the exponent of water, as
+// products with their rounding errors carried along: closer to the exact value
+// than pow, which took 250 instructions a call (an eighth of the FP32
+// water_pass_a's).
+__device__ __forceinline__ double tait(double r, double gamma) {
+    if (gamma == 7.0) {
+        const double r2 = r * r, e2 = fma(r, r, -r2);
+        const double r3 = r2 * r, e3 = fma(r2, r, -r3) + e2 * r;
+        const double r6 = r3 * r3, e6 = fma(r3, r3, -r6) + 2.0 * r3 * e3;
+        const double r7 = r6 * r, e7 = fma(r6, r, -r7) + e6 * r;
+        return (r7 - 1.0) + e7;
+    }
+    return pow(r, gamma) - 1;
+}
+
 // What water_pass_a does with a particle's sums: EOS, newtonian_fluid, the
 // record of the next pass, the interaction count.
 template <typename T, bool SINGLE>
@@ -390,24 +423,26 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
     const int a = P.perm[k];
     T txx, txy, tyy, drho;
     double p, cnew, vof;
+    // every load before the first store
     const double rho = P.rho[a];
+    const int sid = P.sid[a], itype = P.itype[a];
     if (SINGLE) {
+        const double pold = P.p[a];
+        cnew = P.c[a];
         drho = P.drho[a] + dl;
         txx = c23 * (T(2) * t0 - t1);
         txy = t2 + t3;
         tyy = c23 * (T(2) * t1 - t0);
-        p = P.p[a];
-        if (rho > 0.0) p = c.tab[P.sid[a]].w_b * (pow(rho / c.w_rho0, c.w_gamma) - 1);
-        cnew = P.c[a];
+        p = rho > 0.0 ? c.tab[sid].w_b * tait(rho / c.w_rho0, c.w_gamma) : pold;
         vof = 1.0;
     } else {
         drho = con + dl;
         txx = t0; txy = t1; tyy = t2;
         vof = P.vof[a];
         const double ratio = rho / (c.w_rho0 * vof);
-        const SceneTab& st = c.tab[P.sid[a]];
-        p = st.w_b * (pow(ratio, c.w_gamma) - 1);
-        cnew = st.w_c * pow(ratio, 3.0);
+        const SceneTab& st = c.tab[sid];
+        p = st.w_b * tait(ratio, c.w_gamma);
+        cnew = st.w_c * cube(ratio);
         P.c[a] = cnew;
     }
     P.drho[a] = drho;
@@ -418,7 +453,7 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
     RecB<T> rb;
     rb.p = (T)p; rb.c = (T)cnew; rb.vof = (T)vof;
     rb.sxx = (T)sxx; rb.sxy = (T)sxy; rb.syy = (T)syy;
-    rb.itype = (T)P.itype[a]; rb.aux = T(0);
+    rb.itype = (T)itype; rb.aux = T(0);
     P.recB[k] = rb;
     if (!SINGLE) P.countiac[a] = hits;
 }
@@ -579,41 +614,49 @@ __device__ __forceinline__ void water_b_finish(const PhaseDev<T>& P, const GridG
                                                DevCounters* cnt, int k, T rho_a, T phia, const WaterB<T>& w) {
     typedef typename V2<T>::t T2;
     const int a = P.perm[k];
+    Corrector<T> q;
+    T2 av;
+    const int itype = P.itype[a];
+    if (!c.average_velocity) av = P.av[a];
+    if (u.update) q.load(P, a, c, u, false);
+    const bool renorm = !SINGLE && c.volume_fraction && c.renorm_now;
+    double rho = 0.0, vof = 0.0;
+    if (renorm) { rho = P.rho[a]; vof = P.vof[a]; }
     T dvx = w.mx, dvy = w.my;
     if (rho_a > T(0)) { dvx = dvx / rho_a; dvy = dvy / rho_a; }
     dvx = dvx + w.fx;
     dvy = dvy + w.fy + (T)c.gravity;
     if (c.average_velocity) {
-        const bool real_a = P.itype[a] > 0;
-        const T eps = (T)c.epsilon;
-        T2 av; av.x = real_a ? eps * w.xsx : w.xsx; av.y = real_a ? eps * w.xsy : w.xsy;
+        const T eps = itype > 0 ? (T)c.epsilon : T(1);
+        av.x = eps * w.xsx; av.y = eps * w.xsy;
         P.av[a] = av;
     }
-    if constexpr (SINGLE) {
-        T2 o; o.x = dvx; o.y = dvy;
-        P.dv[a] = o;
-        if (u.update) update_one(P, a, c, u.first, 0, 0);   // last pass of the water-only step
-    } else {
+    T2 o; o.x = dvx; o.y = dvy;
+    if constexpr (!SINGLE) {
         const T fd = phia * (T)(-c.numeric_gravity / c.s_perm);
-        T2 o; o.x = dvx + fd * w.cdx; o.y = dvy + fd * w.cdy;
-        P.dv[a] = o;
+        o.x = dvx + fd * w.cdx; o.y = dvy + fd * w.cdy;
+        T dvof = w.dvf;
         if (c.volume_fraction) {
             const T irho0 = (T)(1.0 / c.s_rho0);
-            P.dvof[a] = w.dvf + w.cdvof * irho0;
+            dvof = w.dvf + w.cdvof * irho0;
             const T vof2 = T(1) - w.cv2 * irho0;
             P.vof2[a] = vof2;
-            if (c.renorm_now) {
-                double rho = P.rho[a] / P.vof[a];
-                P.vof[a] = (double)vof2;
-                P.rho[a] = rho * (double)vof2;
+            if (renorm) {
+                rho = rho / vof * (double)vof2;
+                vof = (double)vof2;
+                if (u.first) { q.rho = rho; q.vof = vof; }   // the first step integrates from them
+                if (!u.update) { P.rho[a] = rho; P.vof[a] = vof; }
             }
-        } else {
-            P.dvof[a] = w.dvf;
         }
+        P.dvof[a] = dvof;
         P.countiac[a] = w.chits;
-        if (u.update) update_one(P, a, c, u.first, u.with_vof, 0);   // last pass of the water phase
+        if (u.update && u.with_vof && c.volume_fraction) P.vof[a] = q.vof + (u.first ? q.dt / 2.0 : q.dt) * (double)dvof;
     }
-    if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
+    P.dv[a] = o;
+    double2 xnew;
+    if (u.update) { q.move(P, a, c, u.first, o, av); xnew = q.x; }   // last pass of the water phase
+    else if (u.ncount) xnew = P.x[a];
+    if (u.ncount) cell_key(g, xnew, a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
 }
 
 // ----------------------------------------------------------- water: pass B
@@ -751,26 +794,32 @@ __device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom
                                             int& fail3) {
     typedef typename V2<T>::t T2;
     const int a = P.perm[k];
+    // every load before the first store
+    Corrector<T> cr;
+    T2 av;
+    const int itype = P.itype[a];
+    const double alpha1 = c.tab[P.sid[a]].s_alpha1;
+    const double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
+    const double rho = P.rho[a];
+    if (!c.average_velocity) av = P.av[a];
+    if (u.update) cr.load(P, a, c, u, true);
     T dvx = w.mx, dvy = w.my;
     if (rho_a > T(0)) { dvx = dvx / rho_a; dvy = dvy / rho_a; }
     dvx = dvx + w.fx;
     dvy = dvy + w.fy + (T)c.gravity;
     if (c.average_velocity) {
-        const bool real_a = P.itype[a] > 0;
-        const T eps = (T)c.epsilon;
-        T2 av; av.x = real_a ? eps * w.xsx : w.xsx; av.y = real_a ? eps * w.xsy : w.xsy;
+        const T eps = itype > 0 ? (T)c.epsilon : T(1);
+        av.x = eps * w.xsx; av.y = eps * w.xsy;
         P.av[a] = av;
     }
     P.drho[a] = w.drho;
     // plastic_or_not + plastic_flow_rule3 + Jaumann_rate on the post-DP state
-    const double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
     const double dtxx = (double)w.txx, dtxy = (double)w.txy, dtyy = (double)w.tyy, dvcc = (double)w.vcc;
     const double G = c.s_E / (2.0 * (1 + c.s_niu));
     double ds0 = 0.0, ds1 = 0.0, ds2 = 0.0, dp = 0.0;
     fail = 0;
     if (c.plasticity == 3) {
         const double J2a = sqrt((sxx * sxx + 2.0 * (sxy * sxy) + syy * syy + (sxx + syy) * (sxx + syy)) / 2.0) + 1.0e-6;
-        const double alpha1 = c.tab[P.sid[a]].s_alpha1;
         if (fabs(J2a - alpha1 * (3.0 * p)) < SPHG_F32LIT(1.0e-5f)) fail = 1;
         P.fail[a] = fail;
         if (fail) {
@@ -795,10 +844,9 @@ __device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom
     ds0 = ds0 + 2.0 * sxy * dwxy;
     ds1 = ds1 - (sxx - syy) * dwxy;
     ds2 = ds2 - 2.0 * sxy * dwxy;
-    P.dsxx[a] = (T)(ds0 + (double)w.dsx);
-    P.dsxy[a] = (T)(ds1 + (double)w.dsxy);
-    P.dsyy[a] = (T)(ds2 + (double)w.dsy);
-    P.dp[a] = (T)(dp + (double)w.dp);
+    const T rxx = (T)(ds0 + (double)w.dsx), rxy = (T)(ds1 + (double)w.dsxy), ryy = (T)(ds2 + (double)w.dsy);
+    const T rp = (T)(dp + (double)w.dp);
+    P.dsxx[a] = rxx; P.dsxy[a] = rxy; P.dsyy[a] = ryy; P.dp[a] = rp;
     P.c[a] = c.s_c;
     P.txx[a] = w.txx; P.tyy[a] = w.tyy; P.txy[a] = w.wxy;   // wxy is txy (alias)
     P.vcc[a] = w.vcc;
@@ -808,11 +856,20 @@ __device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom
         const T irs = T(1) / rho_a;
         const T fd = phis * (T)(-c.numeric_gravity / c.s_perm) * irs, fp = irs * phis;
         o.x = dvx + (fd * w.cdx + fp * w.cpx); o.y = dvy + (fd * w.cdy + fp * w.cpy);
-        if (c.volume_fraction) P.vof[a] = P.rho[a] / c.s_rho0;
+        if (c.volume_fraction) P.vof[a] = rho / c.s_rho0;
     }
     P.dv[a] = o;
-    fail3 = u.update ? update_one(P, a, c, u.first, SINGLE ? 0 : u.with_vof, u.do_dp) : 0;   // last pass of the soil phase
-    if (u.ncount) cell_key(g, P.x[a], a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
+    fail3 = 0;
+    double2 xnew;
+    if (u.update) {   // last pass of the soil phase
+        cr.drho = w.drho;
+        cr.move(P, a, c, u.first, o, av);
+        fail3 = cr.stress(P, a, c, u.first, u.do_dp, rxx, rxy, ryy, rp);
+        xnew = cr.x;
+    } else if (u.ncount) {
+        xnew = P.x[a];
+    }
+    if (u.ncount) cell_key(g, xnew, a, P.cell_id, P.cell_fill, u.ncount, cnt, 1);
 }
 
 // ------------------------------------------------------------------ soil
