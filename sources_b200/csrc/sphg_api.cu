@@ -979,11 +979,13 @@ struct Engine : EngineBase {
         u.ncount = nullptr;   // set per phase: the corrector counts that phase's next cells
         const int tpb = SPHG_TPB;
         const int dp = sim.yield_dp;
+        // the paired passes take h from their constants (the water-only step runs the one-particle ones)
+        const int hs = paired() && !(p.single_phase && P[0].material == SPHG_WATER) ? 0 : 1;
         int rc;
         if (p.single_phase) {
             PhaseDev<T>& D = P[0];
             if (D.material == SPHG_WATER) {
-                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 0, 0, fh, 0, 0, cnt))) return rc;
+                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 0, 0, fh, hs, 0, cnt))) return rc;
                 if ((rc = launch_pdl("water_sum", k_water_sum<T, SKF>, blocks(D.n, tpb), tpb, 0, D, grid, sc_same, sim, cnt))) return rc;
                 if ((rc = launch_pdl("water_pass_a", k_water_pass_a<T, SKF, true>, blocks(D.n, tpb), tpb, 0, D, grid, sc_same, sim, cnt))) return rc;
                 StepCtl uw = u;
@@ -991,7 +993,7 @@ struct Engine : EngineBase {
                 if ((rc = launch_pdl("water_pass_b", k_water_pass_b<T, SKF, true, false>, blocks(D.n, tpb), tpb, 0, D, D, grid, sc_same,
                                  sc_same, sim, uw, cnt))) return rc;
             } else {
-                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 1, dp, fh, 0, dp, cnt))) return rc;
+                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 1, dp, fh, hs, dp, cnt))) return rc;
                 StepCtl us = u; us.with_vof = 0; us.do_dp = dp;
                 us.ncount = u.update ? counts[0] : nullptr;
                 if ((rc = launch_soil<SKF, true, false>(D, D, 0, us))) return rc;
@@ -1004,7 +1006,7 @@ struct Engine : EngineBase {
             uw.ncount = u.update ? counts[0] : nullptr;
             us.ncount = u.update ? counts[1] : nullptr;
             // the soil's gather was launched by run() on the side stream
-            if ((rc = launch_pdl("gather", k_gather<T>, blocks(W.n, 256), 256, 0, W, sim, 0, 0, fh, 1, 0, cnt))) return rc;
+            if ((rc = launch_pdl("gather", k_gather<T>, blocks(W.n, 256), 256, 0, W, sim, 0, 0, fh, hs, 0, cnt))) return rc;
             if ((rc = launch_water_a<SKF>(W))) return rc;
             // The cross pairs run inside the last pass of each phase; the soil
             // pass reads the water pressure that water_pass_a sets.  After
@@ -1149,6 +1151,7 @@ struct Engine : EngineBase {
         int rc = prepare();
         if (rc) return rc;
         make_sim(itimestep);
+        sim.half = fh;
         if ((rc = reset_counters())) return rc;
         const sphg_params& p = ctx->prm;
         bool reorder_now = p.reorder_interval > 0 && itimestep > 0 && itimestep % p.reorder_interval == 0;
@@ -1166,8 +1169,8 @@ struct Engine : EngineBase {
             ctx->stream = side;
             rc = build_cells(1);
             if (!rc && reorder_now) rc = reorder(1);
-            if (!rc) rc = launch_pdl("gather", k_gather<T>, blocks(P[1].n, 256), 256, 0, P[1], sim, 1, sim.yield_dp, fh, 1,
-                                 sim.yield_dp, cnt);
+            if (!rc) rc = launch_pdl("gather", k_gather<T>, blocks(P[1].n, 256), 256, 0, P[1], sim, 1, sim.yield_dp, fh,
+                                 paired() ? 0 : 1, sim.yield_dp, cnt);
             cudaError_t ej = side != main_stream ? cudaEventRecord(ctx->ev_join2, side) : cudaSuccess;
             ctx->stream = main_stream;
             if (rc || ej != cudaSuccess) {
@@ -1339,7 +1342,7 @@ struct Engine : EngineBase {
         // step ran since): rebuild sorted positions for both phases
         for (int ph = 0; ph < ctx->nphase; ++ph) {
             if ((rc = build_cells(ph))) { cells_ready = false; return rc; }
-            if ((rc = launch("gather", k_gather<T>, blocks(P[ph].n, 256), 256, P[ph], sim, 0, 0, 0, 0, 0, cnt))) {
+            if ((rc = launch("gather", k_gather<T>, blocks(P[ph].n, 256), 256, P[ph], sim, 0, 0, 0, 1, 0, cnt))) {
                 cells_ready = false;
                 return rc;
             }

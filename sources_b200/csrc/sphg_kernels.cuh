@@ -27,6 +27,7 @@ struct SimConst {
     int skf, single_phase, summation_density, average_velocity, visc_artificial;
     int artificial_density, soil_artificial_stress, volume_fraction, water_artificial_volume;
     int volume_fraction_renorm, stress_integration, plasticity, yield_dp;
+    int half;              // the step starts with the leapfrog predictor (not the first step or a right-hand side alone)
     int renorm_now;        // this step renormalises vof (itimestep % interval == 0)
     double gravity, numeric_gravity, alpha, beta, etq, dd, p1, p2, delta, epsilon, dt;
     double w_rho0, w_b, w_gamma, w_c, w_mu;
@@ -153,43 +154,28 @@ struct StepCtl {
                      // into this phase's per-cell counts for the next step's cell list
 };
 
-// first_half, declarations_sph.f90:643-684 (and :812-825, :998-1025), plus the
-// Drucker-Prager call that follows it on soil (:559, :1027).  Returns the
-// particle's fail flag of that DP call.
+// first_half, declarations_sph.f90:643-684 (and :812-825, :998-1025).  The
+// half-step rho, vof and v are r + dt/2 * rate of the state and the rates of the
+// step before, which stay in place until the corrector; they are formed where
+// they are needed (the gather, water_pass_a, soil_finish) and never stored, and
+// the corrector keeps the full-step values as rho_min, vof_min and v_min.
 template <typename T>
-__device__ __forceinline__ int first_half_one(const PhaseDev<T>& P, int a, const SimConst& c, int with_vof, int do_dp) {
-    const SceneTab& st = c.tab[P.sid[a]];
-    const double dt = st.dt;
-    if (!c.summation_density) { double r = P.rho[a]; P.rho_min[a] = r; P.rho[a] = r + (dt / 2.0) * (double)P.drho[a]; }
-    if (with_vof && P.material == 1 && c.volume_fraction) {
-        double f = P.vof[a]; P.vof_min[a] = f; P.vof[a] = f + (dt / 2.0) * (double)P.dvof[a];
+__device__ __forceinline__ double half_step(double r, double dt, T rate) { return r + (dt / 2.0) * (double)rate; }
+
+// The stress part of first_half on soil (stress_integration 2) and the
+// Drucker-Prager call that follows it (:559, :1027).  Returns its fail flag.
+template <typename T>
+__device__ __forceinline__ int first_half_stress(const PhaseDev<T>& P, int a, const SimConst& c, const SceneTab& st, int do_dp,
+                                                 double& p, double& sxx, double& sxy, double& syy) {
+    if (c.stress_integration == 2) {
+        const T d0 = P.dsxx[a], d1 = P.dsxy[a], d2 = P.dsyy[a], d3 = P.dp[a];
+        P.sxx_min[a] = sxx; P.sxy_min[a] = sxy; P.syy_min[a] = syy; P.p_min[a] = p;
+        sxx = half_step(sxx, st.dt, d0);
+        sxy = half_step(sxy, st.dt, d1);
+        syy = half_step(syy, st.dt, d2);
+        p = half_step(p, st.dt, d3);
     }
-    int fail = 0;
-    const bool soil = P.material == 2;
-    double p = 0, sxx = 0, sxy = 0, syy = 0;
-    if (soil) {
-        p = P.p[a]; sxx = P.sxx[a]; sxy = P.sxy[a]; syy = P.syy[a];
-        if (c.stress_integration == 2) {
-            P.sxx_min[a] = sxx; P.sxy_min[a] = sxy; P.syy_min[a] = syy; P.p_min[a] = p;
-            sxx = sxx + (dt / 2.0) * (double)P.dsxx[a];
-            sxy = sxy + (dt / 2.0) * (double)P.dsxy[a];
-            syy = syy + (dt / 2.0) * (double)P.dsyy[a];
-            p = p + (dt / 2.0) * (double)P.dp[a];
-        }
-    }
-    if (P.itype[a] >= 0) {
-        double2 v = P.v[a];
-        P.v_min[a] = v;
-        const typename V2<T>::t d = P.dv[a];
-        v.x = v.x + (dt / 2.0) * (double)d.x;
-        v.y = v.y + (dt / 2.0) * (double)d.y;
-        P.v[a] = v;
-    }
-    if (soil) {
-        if (do_dp) { fail = dp_return(p, sxx, sxy, syy, st.s_alpha1); P.fail[a] = fail; }
-        P.p[a] = p; P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy;
-    }
-    return fail;
+    return do_dp ? dp_return(p, sxx, sxy, syy, st.s_alpha1) : 0;
 }
 
 // The corrector: first_step (:686-723) when first != 0, else second_half
@@ -209,11 +195,11 @@ struct Corrector {
         const int sid = P.sid[a];
         real = P.itype[a] >= 0;
         x = P.x[a];
-        v = u.first ? P.v[a] : P.v_min[a];
-        rho = u.first ? P.rho[a] : P.rho_min[a];
+        v = P.v[a];
+        rho = c.single_phase && !soil && !u.first ? P.rho_min[a] : P.rho[a];   // the water-only sum has replaced rho
         if (!soil) {
             drho = P.drho[a];
-            vof = u.first ? P.vof[a] : P.vof_min[a];
+            vof = P.vof[a];
         } else if (c.stress_integration == 2 && !u.first) {
             p = P.p_min[a]; sxx = P.sxx_min[a]; sxy = P.sxy_min[a]; syy = P.syy_min[a];
         } else {
@@ -225,8 +211,12 @@ struct Corrector {
     // rho and v, x; the new position
     __device__ __forceinline__ void move(const PhaseDev<T>& P, int a, const SimConst& c, int first, T2 d, T2 av) {
         const double h = first ? dt / 2.0 : dt;
-        if (!c.summation_density) P.rho[a] = rho + h * (double)drho;
+        if (!c.summation_density) {
+            if (!first) P.rho_min[a] = rho;
+            P.rho[a] = rho + h * (double)drho;
+        }
         if (real) {
+            if (!first) P.v_min[a] = v;
             v.x = v.x + h * (double)d.x + (double)av.x;
             x.x = x.x + dt * v.x;
             v.y = v.y + h * (double)d.y + (double)av.y;
@@ -255,40 +245,54 @@ __device__ __forceinline__ void count_fail(DevCounters* cnt, int slot, int fail)
 }
 
 // ------------------------------------------------------------------ gathers
-// Sorted copies of position, h and (v, vol, rho).  With fh != 0 the particle's
-// leapfrog predictor (first_half, + DP on soil) runs first, so the records
-// carry the half-step state.  For soil also the in-step Drucker-Prager return
-// (declarations_sph.f90:1242-1247) on the state and the stress/pressure
-// record of the soil pass.
+// Sorted copies of position, h (with_hs: not needed when every h is equal) and
+// (v, vol, rho).  With fh != 0 the records carry the half-step state of the
+// leapfrog predictor (first_half, + DP on soil).  For soil also the in-step
+// Drucker-Prager return (declarations_sph.f90:1242-1247) on the state and the
+// stress/pressure record of the soil pass.  Bound by DRAM: it reads and writes
+// each field once, with every load before the first store.  Storing the half
+// step as well (and reading it back in the corrector) took 53 us for the two
+// phases of 912,016 particles instead of 34, and the step 345 us instead of
+// 322; 5, 6 and 8 resident blocks spill and take 33, 36 and 38 us.
 template <typename T>
-__global__ void __launch_bounds__(256) k_gather(PhaseDev<T> P, SimConst c, int soil, int do_dp, int fh, int with_vof,
+__global__ void __launch_bounds__(256, 4) k_gather(PhaseDev<T> P, SimConst c, int soil, int do_dp, int fh, int with_hs,
                                                 int fh_dp, DevCounters* cnt) {
     pdl_enter();
     int k = gtid();
     int fail0 = 0, fail = 0;
     if (k < P.n) {
-        int a = P.perm[k];
-        if (fh) fail0 = first_half_one(P, a, c, with_vof, fh_dp);
-        P.xs[k] = P.x[a];
-        P.hs[k] = P.hsml[a];
+        const int a = P.perm[k];
+        const double2 x = P.x[a];
         double2 v = P.v[a];
-        RecA<T> ra;
-        const double rho = P.rho[a];
-        ra.vx = (T)v.x; ra.vy = (T)v.y; ra.vol = (T)(P.mass[a] / rho); ra.rho = (T)rho;
-        P.recA[k] = ra;
+        double rho = P.rho[a];
+        const double mass = P.mass[a], h = with_hs ? P.hsml[a] : 0.0;
+        const int sid = soil || fh ? P.sid[a] : 0, itype = soil || fh ? P.itype[a] : 0;
+        const SceneTab& st = c.tab[sid];
+        double p = 0.0, sxx = 0.0, sxy = 0.0, syy = 0.0, cc = 0.0, vof = 0.0;
+        if (soil) { p = P.p[a]; sxx = P.sxx[a]; sxy = P.sxy[a]; syy = P.syy[a]; cc = P.c[a]; vof = P.vof[a]; }
+        if (fh) {
+            const T drho = P.drho[a];
+            const typename V2<T>::t d = P.dv[a];
+            if (!c.summation_density) rho = half_step(rho, st.dt, drho);
+            if (itype >= 0) { v.x = half_step(v.x, st.dt, d.x); v.y = half_step(v.y, st.dt, d.y); }
+            if (soil) fail0 = first_half_stress(P, a, c, st, fh_dp, p, sxx, sxy, syy);
+        }
         if (soil) {
-            double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
-            if (do_dp) {
-                fail = dp_return(p, sxx, sxy, syy, c.tab[P.sid[a]].s_alpha1);
-                P.p[a] = p; P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy;
-                P.fail[a] = fail;
-            }
+            if (do_dp) fail = dp_return(p, sxx, sxy, syy, st.s_alpha1);
+            if (fh || do_dp) { P.p[a] = p; P.sxx[a] = sxx; P.sxy[a] = sxy; P.syy[a] = syy; }
+            if (do_dp) P.fail[a] = fail;
+            else if (fh && fh_dp) P.fail[a] = fail0;
             RecB<T> rb;
-            rb.p = (T)p; rb.c = (T)P.c[a]; rb.vof = (T)P.vof[a];
+            rb.p = (T)p; rb.c = (T)cc; rb.vof = (T)vof;
             rb.sxx = (T)sxx; rb.sxy = (T)sxy; rb.syy = (T)syy;
-            rb.itype = (T)P.itype[a]; rb.aux = T(0);
+            rb.itype = (T)itype; rb.aux = T(0);
             P.recB[k] = rb;
         }
+        P.xs[k] = x;
+        if (with_hs) P.hs[k] = h;
+        RecA<T> ra;
+        ra.vx = (T)v.x; ra.vy = (T)v.y; ra.vol = (T)(mass / rho); ra.rho = (T)rho;
+        P.recA[k] = ra;
     }
     if (fh && fh_dp) count_fail(cnt, 0, fail0);
     if (soil && do_dp) count_fail(cnt, 1, fail);
@@ -345,14 +349,16 @@ __device__ __forceinline__ void pair_kernel(const KernelConst<T, SKF>& ka, const
 // water-only step, drho = -rho*(df2(vx,'x') + df2(vy,'y'))
 // (declarations_sph.f90:1465-1466, df2 m_particles.f90:1802-1831).
 template <typename T>
-__device__ __forceinline__ void water_sum_finish(const PhaseDev<T>& P, int k, const RecA<T>& ra, T num, T wi, T sx, T sy,
-                                                 int hits) {
+__device__ __forceinline__ void water_sum_finish(const PhaseDev<T>& P, const SimConst& c, int k, const RecA<T>& ra, T num, T wi,
+                                                 T sx, T sy, int hits) {
     const int a = P.perm[k];
     const T rho = num / wi;
+    const double mass = P.mass[a];
+    if (c.half) P.rho_min[a] = P.rho[a];   // the corrector integrates from it
     P.rho[a] = (double)rho;
     P.drho[a] = -rho * (sx / rho + sy / rho);
     RecA<T> r2;
-    r2.vx = ra.vx; r2.vy = ra.vy; r2.vol = (T)(P.mass[a] / (double)rho); r2.rho = rho;
+    r2.vx = ra.vx; r2.vy = ra.vy; r2.vol = (T)(mass / (double)rho); r2.rho = rho;
     P.recA2[k] = r2;
     P.countiac[a] = hits;
 }
@@ -389,7 +395,7 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
     });
     if (valid) {
         if (P.hmask) P.hmask[k] = mask;
-        water_sum_finish(P, k, ra, num, wi, sx, sy, hits);
+        water_sum_finish(P, c, k, ra, num, wi, sx, sy, hits);
     }
     count_stats(cnt, 0, 0, hits, valid);
 }
@@ -424,7 +430,7 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
     T txx, txy, tyy, drho;
     double p, cnew, vof;
     // every load before the first store
-    const double rho = P.rho[a];
+    double rho = P.rho[a];
     const int sid = P.sid[a], itype = P.itype[a];
     if (SINGLE) {
         const double pold = P.p[a];
@@ -439,8 +445,13 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
         drho = con + dl;
         txx = t0; txy = t1; tyy = t2;
         vof = P.vof[a];
-        const double ratio = rho / (c.w_rho0 * vof);
+        const T dold = c.half ? P.drho[a] : T(0), fold = c.half && c.volume_fraction ? P.dvof[a] : T(0);
         const SceneTab& st = c.tab[sid];
+        if (c.half) {
+            rho = half_step(rho, st.dt, dold);
+            if (c.volume_fraction) vof = half_step(vof, st.dt, fold);
+        }
+        const double ratio = rho / (c.w_rho0 * vof);
         p = st.w_b * tait(ratio, c.w_gamma);
         cnew = st.w_c * cube(ratio);
         P.c[a] = cnew;
@@ -650,7 +661,10 @@ __device__ __forceinline__ void water_b_finish(const PhaseDev<T>& P, const GridG
         }
         P.dvof[a] = dvof;
         P.countiac[a] = w.chits;
-        if (u.update && u.with_vof && c.volume_fraction) P.vof[a] = q.vof + (u.first ? q.dt / 2.0 : q.dt) * (double)dvof;
+        if (u.update && u.with_vof && c.volume_fraction) {
+            if (!u.first) P.vof_min[a] = q.vof;
+            P.vof[a] = q.vof + (u.first ? q.dt / 2.0 : q.dt) * (double)dvof;
+        }
     }
     P.dv[a] = o;
     double2 xnew;
@@ -800,7 +814,8 @@ __device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom
     const int itype = P.itype[a];
     const double alpha1 = c.tab[P.sid[a]].s_alpha1;
     const double p = P.p[a], sxx = P.sxx[a], sxy = P.sxy[a], syy = P.syy[a];
-    const double rho = P.rho[a];
+    double rho = P.rho[a];
+    if (c.half) rho = half_step(rho, c.tab[P.sid[a]].dt, P.drho[a]);
     if (!c.average_velocity) av = P.av[a];
     if (u.update) cr.load(P, a, c, u, true);
     T dvx = w.mx, dvy = w.my;
