@@ -167,9 +167,12 @@ void sphg_default_params(sphg_params* p);
 int sphg_create(const sphg_params* p, int n_phase, sphg_ctx** out);
 
 /* Copy one phase (1-based: 1 = `parts`, 2 = `soil`) to the device.  Uploads
- * and downloads go through one device staging area of up to 37 doubles a
+ * and downloads go through one device staging area of up to 39 doubles a
  * particle (at most 512 MB), made at the first transfer of the largest phase
- * and kept until sphg_destroy; pinned host arrays move at the link's speed. */
+ * and kept until sphg_destroy; pinned host arrays move at the link's speed,
+ * pageable ones through page-locked buffers that the contexts share (at most
+ * 8 MB, freed with the last context), with up to three helper threads that
+ * end before the call returns. */
 int sphg_upload_phase(sphg_ctx* ctx, int phase, const sphg_phase_host* v);
 
 /* Right-hand side only: single_step (declarations_sph.f90:1131), or

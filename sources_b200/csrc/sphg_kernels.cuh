@@ -1146,11 +1146,6 @@ __global__ void __launch_bounds__(256) k_from_original(int n, const int* __restr
     S* d = dst + (size_t)a * comps;
     for (int t = 0; t < comps; ++t) d[t] = (S)s[t];
 }
-static __global__ void __launch_bounds__(256) k_to_original_i(int n, const int* __restrict__ orig, const int* __restrict__ src,
-                                                       int* __restrict__ dst) {
-    int a = gtid();
-    if (a < n) dst[orig[a]] = src[a];
-}
 static __global__ void __launch_bounds__(256) k_from_original_i(int n, const int* __restrict__ orig, const int* __restrict__ src,
                                                          int* __restrict__ dst) {
     int a = gtid();
@@ -1159,8 +1154,8 @@ static __global__ void __launch_bounds__(256) k_from_original_i(int n, const int
 
 // Several fields of a phase at once between the state order and the caller's
 // original order, through one staging area in which field i occupies
-// stage[off, off + n*comps) in original order.  wide: the device field is
-// FP64, else of the precision's type S.  One launch per group of fields lets
+// stage[off, off + n*comps) in original order.  wide: 1 the device field is
+// FP64, 0 of the precision's type S, 2 int32 (and int32 in the staging area).  One launch per group of fields lets
 // the host copies of the group run back to back on the copy engine; each
 // field has its own row of blocks (blockIdx.y), so that the fields' loads do
 // not wait on one another.
@@ -1172,6 +1167,7 @@ __global__ void __launch_bounds__(256) k_to_original_all(int n, const int* __res
     const int a = gtid();
     if (a >= n || (int)blockIdx.y >= L.count) return;
     const XferField& f = L.f[blockIdx.y];
+    if (f.wide == 2) { ((int*)(stage + f.off))[orig[a]] = ((const int*)f.dev)[a]; return; }
     double* d = stage + f.off + (size_t)orig[a] * f.comps;
     if (f.wide) {
         const double* s = (const double*)f.dev + (size_t)a * f.comps;
@@ -1204,6 +1200,7 @@ __global__ void __launch_bounds__(256) k_from_original_all(int n, const int* __r
     const int a = gtid();
     if (a >= n || (int)blockIdx.y >= L.count) return;
     const XferField& f = L.f[blockIdx.y];
+    if (f.wide == 2) { ((int*)f.dev)[a] = ((const int*)(stage + f.off))[orig[a]]; return; }
     const double* s = stage + f.off + (size_t)orig[a] * f.comps;
     if (f.wide) {
         double* d = (double*)f.dev + (size_t)a * f.comps;
