@@ -27,15 +27,18 @@ int sphg_gemm_bf16_tn(const void* A, const void* B, float* C, int M, int N, int 
  *   BIAS_ACT  z = acc + bias (z kept when non-null), h = bf16(relu ? max(z, 0) : z)
  *   EDGE      z = acc + bias + P[src[r], :N] + P[dst[r], N:2N] for rows r < nedge
  *             (z kept when non-null), h = bf16(max(z, 0))
- *   RESID     z = z + acc + bias, h = bf16(z) when h is non-null */
-enum { SPHG_EPI_STORE = 0, SPHG_EPI_ACC = 1, SPHG_EPI_BIAS_ACT = 2, SPHG_EPI_EDGE = 3, SPHG_EPI_RESID = 4 };
+ *   RESID     z = z + acc + bias, h = bf16(z) when h is non-null
+ *   RELU_BWD  z = P > 0 ? acc : 0 with P [M x N] the pre-activation (z kept
+ *             when non-null), h = bf16(z) */
+enum { SPHG_EPI_STORE = 0, SPHG_EPI_ACC = 1, SPHG_EPI_BIAS_ACT = 2, SPHG_EPI_EDGE = 3, SPHG_EPI_RESID = 4,
+       SPHG_EPI_RELU_BWD = 5 };
 
 typedef struct SphgGemmEpi {
     int32_t mode, relu;
     const float* bias;   /* [N] */
     float* z;            /* [M x N] fp32 */
     void* h;             /* [M x N] bf16 */
-    const float* P;      /* EDGE: [nodes x 2N] projections gathered per row */
+    const float* P;      /* EDGE: [nodes x 2N] projections gathered per row; RELU_BWD: [M x N] pre-activations */
     const int* src;
     const int* dst;
     long long nedge;
@@ -110,6 +113,15 @@ int sphg_gnn_edge_encoder(const void* F, void* E_out, int M, const void* W1, con
  * up sets *err_dev. */
 int sphg_gnn_node_mlp(const void* X, int M, const void* V1, const float* c1, const void* V2, const float* c2,
                       float* Z, void* H_out, int* err_dev, void* cuda_stream);
+
+/* Weight gradient G[out x in] += Y^T X of the row-major bf16 matrices Y
+ * [rows x out] and X [rows x in], fp32 accumulation, split over the rows (the
+ * partial sums are added to G in no fixed order).  (out, in) in {(128, 64),
+ * (128, 128), (128, 256), (256, 128)} (SPHG_ERR_UNSUPPORTED otherwise), rows %
+ * 128 == 0, 16-byte aligned arrays.  A device wait that gives up sets *err_dev
+ * to 1. */
+int sphg_gnn_wgrad(const void* Y, const void* X, float* G, long long rows, int out, int in, int* err_dev,
+                   void* cuda_stream);
 
 /* Test of the bounded device waits (no counterpart in the reference, whose
  * only failure path is `stop`): launches sphg_gemm_bf16_tn's kernel on
@@ -215,6 +227,30 @@ int sphg_gnn_mse(const float* pred, int ld, const float* target, int nout, const
  * bf16 copy w_bf16 and its transpose wt_bf16 [cols x rows] when non-null */
 int sphg_gnn_adam(float* w, const float* g, float* m, float* v, void* w_bf16, void* wt_bf16, int rows, int cols,
                   float lr, float beta1, float beta2, float eps, int step, int row_limit, void* cuda_stream);
+
+/* The same Adam step of up to SPHG_ADAM_MAX tensors in one launch. */
+enum { SPHG_ADAM_MAX = 56 };
+typedef struct {
+    float *w, *g, *m, *v;
+    void *wb, *wt;               /* bf16 copy and its transpose, or NULL */
+    int32_t rows, cols, row_limit, pad;
+} SphgAdamTensor;
+typedef struct {
+    int32_t count, pad;
+    SphgAdamTensor t[SPHG_ADAM_MAX];
+} SphgAdamList;
+int sphg_gnn_adam_all(const SphgAdamList* list, float lr, float beta1, float beta2, float eps, int step,
+                      void* cuda_stream);
+
+/* y = bf16(x) (skipped when y is NULL) and out[c] += sum_r x[r, c0 + c], c <
+ * 128 (skipped when out is NULL), in one pass; x is [rows x cols], cols 128 or
+ * 256, c0 = 0 or cols - 128. */
+int sphg_gnn_cast_colsum(const float* x, void* y_bf16, long long rows, int cols, int c0, float* out, void* cuda_stream);
+/* de[k] += scale * dagg[dst[k]] for the edges k < nedge (de taken as zero on
+ * entry with init, all npad rows written), de_bf16 = bf16(de), gbias[c] +=
+ * sum_k de[k, c]; rows of 128 */
+int sphg_gnn_edge_grad(const float* dagg, const int* dst, float* de, void* de_bf16, float* gbias, long long nedge,
+                       long long npad, float scale, int init, void* cuda_stream);
 
 /* learned stride: a = pred[:, :2] * norm[2:4] + norm[0:2]; v' = v + a dts;
  * x += v' dts clamped to the walls (margin); v' -> slot head_new */

@@ -275,6 +275,61 @@ __global__ void k_colsum(const float* __restrict__ x, long long rows, int cols, 
     atomicAdd(out + c, s);
 }
 
+// Sums of the block's rows of 128 columns (4 per lane, 8 rows at a time) added
+// to out[128]: partial sums per warp, through shared memory.
+__device__ __forceinline__ void add_block_colsum(float4 s, float* __restrict__ out) {
+    __shared__ float4 part[8][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    part[w][lane] = s;
+    __syncthreads();
+    if (threadIdx.x < 128) {
+        const float* f = reinterpret_cast<const float*>(part);
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += f[i * 128 + threadIdx.x];
+        atomicAdd(out + threadIdx.x, t);
+    }
+}
+
+// y = bf16(x) (when y is not null) and out[c] += column sums of columns c0 ..
+// c0 + 127, in one pass over x [rows x cols], cols 128 or 256: one warp per 128
+// columns of a row, grid-stride over the rows.
+__global__ void __launch_bounds__(256) k_cast_colsum(const float4* __restrict__ x, uint2* __restrict__ y, long long rows, int q4,
+                                                     int c0q, float* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int halves = q4 / 32;
+    for (long long u = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); u < rows * halves; u += (long long)gridDim.x * 8) {
+        const long long i = u * 32 + lane;
+        const float4 v = x[i];
+        if (y) y[i] = pack4(v);
+        if (halves == 1 || (int)(u % halves) * 32 == c0q) s = add4(s, v);
+    }
+    if (out) add_block_colsum(s, out);
+}
+
+// The gradient of the edge rows that enters an edge layer's backward pass, in one
+// pass: de += scale * dagg[dst] (rows below nedge; de starts from zero with
+// init), its bf16 copy, and the column sums (the gradient of b2).
+__global__ void __launch_bounds__(256) k_edge_grad(const float* __restrict__ dagg, const int* __restrict__ dst,
+                                                   float4* __restrict__ de, uint2* __restrict__ deb, float* __restrict__ gb,
+                                                   long long nedge, long long npad, float scale, int init) {
+    const int lane = threadIdx.x & 31;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long k = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); k < npad; k += (long long)gridDim.x * 8) {
+        const long long i = k * 32 + lane;
+        float4 d = init ? make_float4(0.f, 0.f, 0.f, 0.f) : de[i];
+        if (k < nedge) {
+            const float4 g = reinterpret_cast<const float4*>(dagg + (long long)dst[k] * LW)[lane];
+            d = add4(d, make_float4(g.x * scale, g.y * scale, g.z * scale, g.w * scale));
+        }
+        de[i] = d;
+        deb[i] = pack4(d);
+        s = add4(s, d);
+    }
+    add_block_colsum(s, gb);
+}
+
 // out[c, r] = in[r, c] in bf16 (32 x 32 tiles through shared memory)
 template <typename S>
 __global__ void k_transpose(const S* __restrict__ in, bf16* __restrict__ out, long long rows, int cols) {
@@ -387,10 +442,8 @@ __global__ void k_gather_bwd_src(const float* __restrict__ dz, const int* __rest
     if (k >= nedge) return;
     const float4 g = reinterpret_cast<const float4*>(dz + k * LW)[lane];
     float* d = dP + (long long)src[k] * 2 * LW + lane * 4;
-    atomicAdd(d, g.x);
-    atomicAdd(d + 1, g.y);
-    atomicAdd(d + 2, g.z);
-    atomicAdd(d + 3, g.w);
+    // one 16-byte reduction instead of four atomics
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(g.x), "f"(g.y), "f"(g.z), "f"(g.w) : "memory");
 }
 
 // [h | agg] as bf16 rows of 2L: 16 bytes (8 values) per thread
@@ -474,6 +527,29 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
     w[i] = wi;
     if (wb) wb[i] = __float2bfloat16_rn(wi);
     if (wt) wt[(long long)c * rows + r] = __float2bfloat16_rn(wi);
+}
+
+// The same step of every tensor of the network in one launch: blockIdx.y picks
+// the tensor.
+__global__ void __launch_bounds__(256) k_adam_all(const __grid_constant__ SphgAdamList L, float lr, float b1, float b2, float eps,
+                                                  float c1, float c2) {
+    const SphgAdamTensor& T = L.t[blockIdx.y];
+    const int n = T.rows * T.cols;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const int r = i / T.cols, c = i - r * T.cols;
+        float wi = 0.f;
+        if (r < T.row_limit) {
+            const float gi = T.g[i];
+            const float mi = b1 * T.m[i] + (1.f - b1) * gi;
+            const float vi = b2 * T.v[i] + (1.f - b2) * gi * gi;
+            T.m[i] = mi;
+            T.v[i] = vi;
+            wi = T.w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        }
+        T.w[i] = wi;
+        if (T.wb) static_cast<bf16*>(T.wb)[i] = __float2bfloat16_rn(wi);
+        if (T.wt) static_cast<bf16*>(T.wt)[(long long)c * T.rows + r] = __float2bfloat16_rn(wi);
+    }
 }
 
 // ---------------------------------------------------------------- rollout
@@ -653,6 +729,36 @@ int sphg_gnn_colsum(const float* x, long long rows, int cols, float* out, void* 
     if (rows <= 0 || cols <= 0) return SPHG_OK;
     dim3 grid(nb(rows, 512), nb(cols, 128));
     k_colsum<<<grid, 128, 0, (cudaStream_t)stream>>>(x, rows, cols, out);
+    return ok_or_cuda();
+}
+
+// blocks of a grid-stride pass over `rows` rows, 8 at a time
+inline unsigned stride_blocks(long long rows) { const long long b = (rows + 63) / 64; return (unsigned)(b < 1184 ? (b < 1 ? 1 : b) : 1184); }
+
+int sphg_gnn_cast_colsum(const float* x, void* y, long long rows, int cols, int c0, float* out, void* stream) {
+    if (!x || rows <= 0 || (cols != LW && cols != 2 * LW) || (c0 != 0 && c0 != cols - LW)) return SPHG_ERR_BAD_ARG;
+    k_cast_colsum<<<stride_blocks(rows), 256, 0, (cudaStream_t)stream>>>((const float4*)x, (uint2*)y, rows, cols / 4, c0 / 4, out);
+    return ok_or_cuda();
+}
+
+int sphg_gnn_edge_grad(const float* dagg, const int* dst, float* de, void* deb, float* gbias, long long nedge,
+                       long long npad, float scale, int init, void* stream) {
+    if (!dagg || !dst || !de || !deb || !gbias || npad < nedge || npad <= 0) return SPHG_ERR_BAD_ARG;
+    k_edge_grad<<<stride_blocks(npad), 256, 0, (cudaStream_t)stream>>>(dagg, dst, (float4*)de, (uint2*)deb, gbias, nedge, npad,
+                                                                      scale, init);
+    return ok_or_cuda();
+}
+
+int sphg_gnn_adam_all(const SphgAdamList* list, float lr, float b1, float b2, float eps, int step, void* stream) {
+    if (!list || step < 1 || list->count < 1 || list->count > SPHG_ADAM_MAX) return SPHG_ERR_BAD_ARG;
+    int most = 0;
+    for (int i = 0; i < list->count; ++i) {
+        const SphgAdamTensor& t = list->t[i];
+        if (!t.w || !t.g || !t.m || !t.v || t.rows < 1 || t.cols < 1) return SPHG_ERR_BAD_ARG;
+        most = t.rows * t.cols > most ? t.rows * t.cols : most;
+    }
+    const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
+    k_adam_all<<<dim3(nb(most, 1024), (unsigned)list->count), 256, 0, (cudaStream_t)stream>>>(*list, lr, b1, b2, eps, c1, c2);
     return ok_or_cuda();
 }
 

@@ -213,6 +213,8 @@ int launch_gemm(const __nv_bfloat16* A, const __nv_bfloat16* B, float* C, int M,
 //   EDGE      z = acc + bias + P[src[row], :N] + P[dst[row], N:] (rows < nedge),
 //             h = bf16(relu(z))
 //   RESID     z = z + acc + bias, h = bf16(z) when h != null
+//   RELU_BWD  z = P > 0 ? acc : 0 (kept when z != null), h = bf16(z): the
+//             gradient at a ReLU's input from its pre-activation P [M x N]
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -288,7 +290,8 @@ __device__ __forceinline__ void ws_epilogue_staged(const SphgGemmEpi& ep, uint32
     const int q = lane & 3, rs = lane >> 2;   // this lane's 16-byte unit, and its row within each group of 8
     const int mode = MODE >= 0 ? MODE : ep.mode;
     const bool readz = mode == SPHG_EPI_ACC || mode == SPHG_EPI_RESID;
-    const bool bias = mode != SPHG_EPI_STORE && mode != SPHG_EPI_ACC;
+    const bool mask = mode == SPHG_EPI_RELU_BWD;
+    const bool bias = mode != SPHG_EPI_STORE && mode != SPHG_EPI_ACC && !mask;
     const bool hout = mode != SPHG_EPI_STORE && mode != SPHG_EPI_ACC && (ep.h || hs);
     const bool act = mode == SPHG_EPI_EDGE || (mode == SPHG_EPI_BIAS_ACT && ep.relu);
     bool edge[4];
@@ -313,6 +316,7 @@ __device__ __forceinline__ void ws_epilogue_staged(const SphgGemmEpi& ep, uint32
         const int col = cc + 4 * q;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
+            if (mask) zf[i] = reinterpret_cast<const float4*>(ep.P + (row0 + 8 * i + rs) * N)[col / 4];
             if (readz) {
                 if (ep.z) zf[i] = reinterpret_cast<const float4*>(ep.z + (row0 + 8 * i + rs) * N)[col / 4];
                 else zh[i] = reinterpret_cast<const uint2*>(zb + (row0 + 8 * i + rs) * N)[col / 4];
@@ -328,7 +332,7 @@ __device__ __forceinline__ void ws_epilogue_staged(const SphgGemmEpi& ep, uint32
         float4 add[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            add[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            add[i] = mask ? zf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
             if (readz) {
                 if (ep.z) {
                     add[i] = zf[i];
@@ -356,6 +360,10 @@ __device__ __forceinline__ void ws_epilogue_staged(const SphgGemmEpi& ep, uint32
             const int r = 8 * i + rs;
             const float4 a = stage[r * 4 + (q ^ ((r >> 1) & 3))];
             float o[4] = {a.x + add[i].x, a.y + add[i].y, a.z + add[i].z, a.w + add[i].w};
+            if (mask) {
+                o[0] = add[i].x > 0.f ? a.x : 0.f; o[1] = add[i].y > 0.f ? a.y : 0.f;
+                o[2] = add[i].z > 0.f ? a.z : 0.f; o[3] = add[i].w > 0.f ? a.w : 0.f;
+            }
             const long long grow = row0 + r;
             if (ep.z) reinterpret_cast<float4*>(ep.z + grow * N)[col / 4] = make_float4(o[0], o[1], o[2], o[3]);
             if (hout) {
@@ -530,6 +538,7 @@ int launch_ws(const __nv_bfloat16* A, const __nv_bfloat16* B, int M, const SphgG
         case SPHG_EPI_ACC: return launch_ws_mode<N, K, SPHG_EPI_ACC>(A, B, M, ep, err, s);
         case SPHG_EPI_BIAS_ACT: return launch_ws_mode<N, K, SPHG_EPI_BIAS_ACT>(A, B, M, ep, err, s);
         case SPHG_EPI_EDGE: return launch_ws_mode<N, K, SPHG_EPI_EDGE>(A, B, M, ep, err, s);
+        case SPHG_EPI_RELU_BWD: return launch_ws_mode<N, K, SPHG_EPI_RELU_BWD>(A, B, M, ep, err, s);
         default: return launch_ws_mode<N, K, SPHG_EPI_RESID>(A, B, M, ep, err, s);
     }
 }
@@ -1279,6 +1288,151 @@ __global__ void __launch_bounds__(EdgeNodeShape::THREADS, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
+// ------------------------------------------------------------------------
+// Weight gradient dW[OUT x IN] += Y^T X of the row-major bf16 matrices Y
+// [rows x OUT] and X [rows x IN]: the reduction runs down the rows, so both
+// operands are MN-major (the contiguous index is M or N, not K) and go to the
+// tensor cores as they lie in memory, with no transposed copies.  TMA boxes of 64
+// columns x 64 rows in the 128-byte swizzle; a box is eight 8-row atoms, SBO =
+// 1024 bytes apart along K, and the next 64 columns are LBO = 8192 bytes on.
+// Split over the CTAs by rows; each keeps its partial sum in TMEM and adds it
+// to dW once (red.global.add.v4.f32).  Bound by HBM: each row is read once.
+// At 430k edge rows the 128 x 128 gradient takes 40 us (5.5 TB/s); two transposes and
+// the split-K GEMM of k_gemm_bf16_tn took 138 + 120 + 172 us.
+// Warp 0's lane 0 loads a ring of NST row blocks, warp 1's lane 0 issues the
+// MMAs, all four warps read the accumulator out.  Every wait is bounded: on
+// timeout the kernel sets *err, waits (bounded) for its copies and MMAs in
+// flight, frees TMEM and returns.
+template <int OUT, int IN>
+struct WgShape {
+    static constexpr int RT = 64;                        // rows per ring slot
+    static constexpr uint32_t BOX = RT * 128;            // 64 columns x RT rows
+    static constexpr uint32_t SLOT = (OUT + IN) / 64 * BOX;
+    static constexpr int NST = 4;
+    static constexpr uint32_t BAR = NST * SLOT;
+    static constexpr uint32_t SMEM = BAR + 128 + 1024;   // + alignment of the ring to 1024 bytes
+    static constexpr int TCOLS = OUT / 128 * IN;
+};
+
+// K-step descriptor of an MN-major operand in the 128-byte swizzle (above)
+__device__ __forceinline__ uint64_t make_desc_mn128(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)(8192 >> 4) << 16;    // leading byte offset: the next 64 columns
+    d |= (uint64_t)(1024 >> 4) << 32;    // stride byte offset: the next 8 rows
+    d |= (uint64_t)1 << 46;              // version
+    d |= (uint64_t)2 << 61;              // SWIZZLE_128B
+    return d;
+}
+
+template <int OUT, int IN>
+__global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmX,
+                                                  float* __restrict__ G, int nblk, int* __restrict__ err) {
+    typedef WgShape<OUT, IN> S;
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* sm = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+    uint64_t* full = (uint64_t*)(sm + S::BAR);
+    uint64_t* empty = full + S::NST;
+    uint64_t* done = empty + S::NST;
+    uint32_t* tslot = (uint32_t*)(done + 1);
+    volatile int* abort_flag = (volatile int*)(tslot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b0 = (int)((long long)nblk * blockIdx.x / gridDim.x), b1 = (int)((long long)nblk * (blockIdx.x + 1) / gridDim.x);
+    const int my = b1 - b0;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                     "r"(S::TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (tid == 0) {
+        for (int s = 0; s < S::NST; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(full + s)), "r"(1));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(empty + s)), "r"(1));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(done)), "r"(1));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::);
+        *abort_flag = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::);
+    const uint32_t tmem = *tslot;
+    auto fail = [&]() { atomicOr(err, 1); *abort_flag = 1; };
+
+    if (warp == 0 && lane == 0) {
+        int i = 0;
+        for (; i < my; ++i) {
+            const int s = i % S::NST;
+            if (i >= S::NST && (*abort_flag ||
+                                !mbar_wait(smem_u32(empty + s), (uint32_t)(((i / S::NST) & 1) ^ 1), kWaitLimit))) {
+                fail();
+                break;
+            }
+            const uint32_t slot = smem_u32(sm + s * S::SLOT), fb = smem_u32(full + s);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(S::SLOT) : "memory");
+#pragma unroll
+            for (int b = 0; b < (OUT + IN) / 64; ++b) {
+                const CUtensorMap* m = b < OUT / 64 ? &tmY : &tmX;
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                    " [%0], [%1, {%2, %3}], [%4];" ::"r"(slot + b * S::BOX), "l"(m), "r"((b < OUT / 64 ? b : b - OUT / 64) * 64),
+                    "r"((b0 + i) * S::RT), "r"(fb)
+                    : "memory");
+            }
+        }
+        if (i < my)   // copies in flight end before the ring is given back
+            for (int j = i > S::NST ? i - S::NST : 0; j < i; ++j)
+                mbar_wait(smem_u32(full + j % S::NST), (uint32_t)((j / S::NST) & 1), kWaitLimit);
+    } else if (warp == 1 && lane == 0) {
+        // A and B bf16, both MN-major (bits 15 and 16)
+        const uint32_t idesc = make_idesc(IN) | (1u << 15) | (1u << 16);
+        int i = 0;
+        for (; i < my; ++i) {
+            const int s = i % S::NST;
+            if (*abort_flag || !mbar_wait(smem_u32(full + s), (uint32_t)((i / S::NST) & 1), kWaitLimit)) {
+                fail();
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::);
+            const uint32_t a = smem_u32(sm + s * S::SLOT), b = a + OUT / 64 * S::BOX;
+#pragma unroll
+            for (int kk = 0; kk < S::RT / 16; ++kk)   // 16 rows are 2048 bytes into every box
+#pragma unroll
+                for (int h = 0; h < OUT / 128; ++h)
+                    umma_f16(tmem + (uint32_t)(h * IN), make_desc_mn128(a + h * 2 * S::BOX + kk * 2048),
+                             make_desc_mn128(b + kk * 2048), idesc, (i | kk) != 0 ? 1u : 0u);
+            umma_commit(empty + s);
+        }
+        umma_commit(done);   // completes when every MMA issued above has
+    }
+    bool ok = mbar_wait(smem_u32(done), 0u, kWaitLimit);
+    __syncwarp();
+    if (!ok) fail();
+    ok = __syncthreads_and(ok && !*abort_flag) != 0;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::);
+    if (ok && my > 0) {
+#pragma unroll 1
+        for (int h = 0; h < OUT / 128; ++h) {
+            float* row = G + (size_t)(h * 128 + warp * 32 + lane) * IN;
+            const uint32_t t = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * IN);
+#pragma unroll 1
+            for (int c = 0; c < IN; c += 16) {
+                float v[16];
+                tmem_ld16(t + (uint32_t)c, v);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + c + 4 * q), "f"(v[4 * q]),
+                                 "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                                 : "memory");
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::);
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TCOLS));
+}
+
 }  // namespace
 
 // cuTensorMapEncodeTiled from the driver, through the runtime (no link to libcuda)
@@ -1304,6 +1458,41 @@ static CUresult encode_tiled(CUtensorMap* map, const void* base, uint64_t rows, 
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+template <int OUT, int IN>
+static int launch_wgrad(const void* Y, const void* X, float* G, long long rows, int* err, cudaStream_t s) {
+    typedef WgShape<OUT, IN> S;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(k_wgrad<OUT, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM) != cudaSuccess)
+            return SPHG_ERR_CUDA;
+        configured = true;
+    }
+    CUtensorMap tmY, tmX;
+    if (encode_tiled(&tmY, Y, (uint64_t)rows, S::RT, OUT) != CUDA_SUCCESS ||
+        encode_tiled(&tmX, X, (uint64_t)rows, S::RT, IN) != CUDA_SUCCESS)
+        return SPHG_ERR_CUDA;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int nblk = (int)(rows / S::RT);
+    // a CTA's share pays for adding OUT x IN sums: at least four row blocks each
+    const int grid = nblk < 4 ? 1 : nblk / 4 < sms ? nblk / 4 : sms;
+    k_wgrad<OUT, IN><<<grid, 128, S::SMEM, s>>>(tmY, tmX, G, nblk, err);
+    return cudaGetLastError() == cudaSuccess ? SPHG_OK : SPHG_ERR_CUDA;
+}
+
+extern "C" int sphg_gnn_wgrad(const void* Y, const void* X, float* G, long long rows, int out, int in, int* err_dev,
+                              void* stream) {
+    if (!Y || !X || !G || !err_dev || rows <= 0 || rows % 128 || rows >= (1LL << 31)) return SPHG_ERR_BAD_ARG;
+    if (((uintptr_t)Y | (uintptr_t)X | (uintptr_t)G) & 15) return SPHG_ERR_BAD_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (out == 128 && in == 64) return launch_wgrad<128, 64>(Y, X, G, rows, err_dev, s);
+    if (out == 128 && in == 128) return launch_wgrad<128, 128>(Y, X, G, rows, err_dev, s);
+    if (out == 128 && in == 256) return launch_wgrad<128, 256>(Y, X, G, rows, err_dev, s);
+    if (out == 256 && in == 128) return launch_wgrad<256, 128>(Y, X, G, rows, err_dev, s);
+    return SPHG_ERR_UNSUPPORTED;
 }
 
 extern "C" int sphg_gnn_edge_layer_nodes(const void* E, void* E_out, const void* H, const float* Pd, int nnode,
@@ -1428,9 +1617,11 @@ extern "C" int sphg_gemm_bf16_ws(const void* A, const void* B, int M, int N, int
     if (!A || !B || !epi || !err_dev || M <= 0 || M % 128) return SPHG_ERR_BAD_ARG;
     if ((((uintptr_t)A) | ((uintptr_t)B)) & 15) return SPHG_ERR_BAD_ARG;
     const SphgGemmEpi& e = *epi;
-    if (e.mode < SPHG_EPI_STORE || e.mode > SPHG_EPI_RESID) return SPHG_ERR_BAD_ARG;
+    if (e.mode < SPHG_EPI_STORE || e.mode > SPHG_EPI_RELU_BWD) return SPHG_ERR_BAD_ARG;
     const bool need_z = e.mode == SPHG_EPI_STORE || e.mode == SPHG_EPI_ACC || e.mode == SPHG_EPI_RESID;
-    if ((need_z && !e.z) || (e.mode != SPHG_EPI_STORE && e.mode != SPHG_EPI_ACC && !e.bias)) return SPHG_ERR_BAD_ARG;
+    const bool relu_bwd = e.mode == SPHG_EPI_RELU_BWD;
+    if ((need_z && !e.z) || (e.mode != SPHG_EPI_STORE && e.mode != SPHG_EPI_ACC && !relu_bwd && !e.bias)) return SPHG_ERR_BAD_ARG;
+    if (relu_bwd && (!e.P || !e.h)) return SPHG_ERR_BAD_ARG;
     if (e.mode == SPHG_EPI_EDGE && (!e.P || !e.src || !e.dst || !e.h || e.nedge < 0 || e.nedge > M))
         return SPHG_ERR_BAD_ARG;
     if ((((uintptr_t)e.z) | ((uintptr_t)e.h) | ((uintptr_t)e.bias) | ((uintptr_t)e.P)) & 15) return SPHG_ERR_BAD_ARG;

@@ -75,7 +75,18 @@ class GemmEpi(C.Structure):
                 ("nedge", C.c_longlong)]
 
 
-EPI_STORE, EPI_ACC, EPI_BIAS_ACT, EPI_EDGE, EPI_RESID = range(5)
+EPI_STORE, EPI_ACC, EPI_BIAS_ACT, EPI_EDGE, EPI_RESID, EPI_RELU_BWD = range(6)
+ADAM_MAX = 56
+
+
+class AdamTensor(C.Structure):
+    """SphgAdamTensor (include/sphg_learn.h)."""
+    _fields_ = [(n, C.c_void_p) for n in ("w", "g", "m", "v", "wb", "wt")] + [
+        (n, C.c_int32) for n in ("rows", "cols", "row_limit", "pad")]
+
+
+class AdamList(C.Structure):
+    _fields_ = [("count", C.c_int32), ("pad", C.c_int32), ("t", AdamTensor * ADAM_MAX)]
 
 
 class Grid(C.Structure):
@@ -218,16 +229,24 @@ class MPNet:
         w = weights if weights is not None else init_weights(seed)
         self.W, self.B = {}, {}
         Ws, Bs = weight_specs()
+        # every gradient in one buffer, cleared at once
+        self.grads = t.zeros(sum(r * c for _, r, c, _ in Ws) + sum(r for _, r, _ in Bs), dtype=t.float32,
+                             device=self.device)
+        taken = 0
         for name, r, c, lim in Ws:
             m = t.from_numpy(np.ascontiguousarray(w[name], dtype=np.float32)).to(self.device)
-            self.W[name] = dict(w=m, wb=m.to(t.bfloat16), wt=m.t().contiguous().to(t.bfloat16), g=t.zeros_like(m),
+            self.W[name] = dict(w=m, wb=m.to(t.bfloat16), wt=m.t().contiguous().to(t.bfloat16),
+                                g=self.grads[taken:taken + r * c].view(r, c),
                                 m=t.zeros_like(m), v=t.zeros_like(m), rows=r, cols=c, lim=lim)
+            taken += r * c
         for name, r, lim in Bs:
             m = t.from_numpy(np.ascontiguousarray(w[name], dtype=np.float32)).to(self.device)
-            self.B[name] = dict(w=m, g=t.zeros_like(m), m=t.zeros_like(m), v=t.zeros_like(m), rows=r, lim=lim)
+            self.B[name] = dict(w=m, g=self.grads[taken:taken + r], m=t.zeros_like(m), v=t.zeros_like(m), rows=r, lim=lim)
+            taken += r
         self.err = t.zeros(1, dtype=t.int32, device=self.device)
         self.loss_buf = t.zeros(1, dtype=t.float32, device=self.device)
         self.adam_step = 0
+        self.adam_list = None    # the tensors of sphg_gnn_adam_all, made at the first step
         # inputs include the displacement since the reference positions
         self.use_x0 = True
         # normalisation: velocity scale, acceleration mean (2) and std (2)
@@ -269,17 +288,6 @@ class MPNet:
         net.norm.copy_(net.torch.from_numpy(np.asarray(d["_norm"], np.float32)))
         return net
 
-    def _gemm(self, A, B, Cm, M, N, K, acc=0, split=1):
-        self.launches += 1
-        _call(self.L.sphg_gemm_bf16_tn(_ptr(A), _ptr(B), _ptr(Cm), M, N, K, acc, split, _ptr(self.err), self.stream),
-              "sphg_gemm_bf16_tn")
-
-    @staticmethod
-    def _split(M, N, K):
-        bn = 128 if N % 128 == 0 else 64 if N % 64 == 0 else 32 if N % 32 == 0 else 16
-        tiles = (M // 128) * (N // bn)
-        return max(1, min(K // 64 // 2, (2 * 148) // max(tiles, 1)))
-
     def _ws(self, X, Wm, rows, N, K, mode, relu=0, bias=None, z=None, h=None, P=None, src=None, dst=None, nedge=0):
         """Weight-stationary GEMM X [rows x K] . Wm[N x K]^T with a fused epilogue."""
         e = GemmEpi(mode, relu, _ptr(bias), _ptr(z), _ptr(h), _ptr(P), _ptr(src), _ptr(dst), nedge)
@@ -291,24 +299,16 @@ class MPNet:
         self.launches += 1
         _call(getattr(self.L, fn)(*args), fn)
 
-    def _wgrad(self, dY, X, name, rows):
-        """W.g += dY^T X through two transposes and one split-K GEMM."""
-        t = self.torch
+    def _wgrad(self, dYb, X, name, rows):
+        """W.g += dY^T X of bf16 rows."""
         w = self.W[name]
-        out, inn = w["rows"], w["cols"]
-        tA = self.bufs.get("tA", (out, rows), t.bfloat16)
-        tB = self.bufs.get("tB", (inn, rows), t.bfloat16)
-        self._k("sphg_gnn_transpose", _ptr(dY), 1 if dY.dtype == t.float32 else 0, _ptr(tA), rows, out, self.stream)
-        self._k("sphg_gnn_transpose", _ptr(X), 1 if X.dtype == t.float32 else 0, _ptr(tB), rows, inn, self.stream)
-        self._gemm(tA, tB, w["g"], out, inn, rows, acc=1, split=self._split(out, inn, rows))
+        self._k("sphg_gnn_wgrad", _ptr(dYb), _ptr(X), _ptr(w["g"]), rows, w["rows"], w["cols"], _ptr(self.err), self.stream)
 
-    def _bgrad(self, dY, bname, rows):
-        self._k("sphg_gnn_colsum", _ptr(dY), rows, dY.shape[1], _ptr(self.B[bname]["g"]), self.stream)
-
-    def _bf16(self, x, name):
-        t = self.torch
-        y = self.bufs.get(name, tuple(x.shape), t.bfloat16)
-        self._k("sphg_gnn_f32_to_bf16", _ptr(x), _ptr(y), x.numel(), self.stream)
+    def _cast_bgrad(self, dY, bname, name=None):
+        """B.g += the column sums of fp32 dY (of its last 128 columns) and, given a buffer name, dY's bf16 copy."""
+        rows, cols = dY.shape
+        y = self.bufs.get(name, (rows, cols), self.torch.bfloat16) if name else None
+        self._k("sphg_gnn_cast_colsum", _ptr(dY), _ptr(y), rows, cols, cols - L_WIDTH, _ptr(self.B[bname]["g"]), self.stream)
         return y
 
     # ------------------------------------------------------------- forward
@@ -398,8 +398,7 @@ class MPNet:
 
     # ------------------------------------------------------------ backward
     def zero_grad(self):
-        for d in list(self.W.values()) + list(self.B.values()):
-            d["g"].zero_()
+        self.grads.zero_()
 
     def loss(self, b: Batch, out, delta: float = 0.0):
         """Masked mean squared error over the 2 acceleration columns (Huber
@@ -432,21 +431,19 @@ class MPNet:
         Np, Ep = b.n_pad, b.E_pad
         s = self.stream
         # decoder
-        self._bgrad(dout, "dec.b2", Np)
-        self._wgrad(dout, G("dua", (Np, L), bf), "dec.w2", Np)
-        tmpN = G("tmpN", (Np, L), f32)
-        self._ws(self._bf16(dout, "doutb"), self.W["dec.w2"]["wt"], Np, L, L, EPI_STORE, z=tmpN)
+        doutb = self._cast_bgrad(dout, "dec.b2", "doutb")
+        self._wgrad(doutb, G("dua", (Np, L), bf), "dec.w2", Np)
         dy = G("dy", (Np, L), f32)
         dyb = G("dyb", (Np, L), bf)
-        self._k("sphg_gnn_relu_bwd", _ptr(tmpN), _ptr(G("du", (Np, L), f32)), _ptr(dy), _ptr(dyb), Np * L, s)
-        self._bgrad(dy, "dec.b1", Np)
-        self._wgrad(dy, G(f"hb{LAYERS}", (Np, L), bf), "dec.w1", Np)
+        self._ws(doutb, self.W["dec.w2"]["wt"], Np, L, L, EPI_RELU_BWD, z=dy, h=dyb, P=G("du", (Np, L), f32))
+        self._cast_bgrad(dy, "dec.b1")
+        self._wgrad(dyb, G(f"hb{LAYERS}", (Np, L), bf), "dec.w1", Np)
         dh = G("dh", (Np, L), f32)
         self._ws(dyb, self.W["dec.w1"]["wt"], Np, L, L, EPI_STORE, z=dh)
-        de = G("de", (Ep, L), f32, zero=True)
+        de = G("de", (Ep, L), f32, zero=trace is not None)   # else the last layer's edge_grad starts it
+        deb = G("deb", (Ep, L), bf)
         dcat = G("dcat", (Np, 2 * L), f32)
         dagg = G("dagg", (Np, L), f32)
-        da = G("da", (Ep, L), f32)
         dz = G("dz", (Ep, L), f32)
         dzb = G("dzb", (Ep, L), bf)
         dP = G("dP", (Np, 2 * L), f32)
@@ -458,53 +455,47 @@ class MPNet:
             z, a = G(f"z{l}", (Ep, L), f32), G(f"a{l}", (Ep, L), bf)
             y, ya, cat = G(f"y{l}", (Np, L), f32), G(f"ya{l}", (Np, L), bf), G(f"cat{l}", (Np, 2 * L), bf)
             # node update h' = h + relu(y) V2^T + c2
-            self._bgrad(dh, p + "c2", Np)
-            self._wgrad(dh, ya, p + "v2", Np)
-            self._ws(self._bf16(dh, "dhb"), self.W[p + "v2"]["wt"], Np, L, L, EPI_STORE, z=tmpN)
-            self._k("sphg_gnn_relu_bwd", _ptr(tmpN), _ptr(y), _ptr(dy), _ptr(dyb), Np * L, s)
-            self._bgrad(dy, p + "c1", Np)
-            self._wgrad(dy, cat, p + "v1", Np)
+            dhb = self._cast_bgrad(dh, p + "c2", "dhb")
+            self._wgrad(dhb, ya, p + "v2", Np)
+            self._ws(dhb, self.W[p + "v2"]["wt"], Np, L, L, EPI_RELU_BWD, z=dy, h=dyb, P=y)
+            self._cast_bgrad(dy, p + "c1")
+            self._wgrad(dyb, cat, p + "v1", Np)
             self._ws(dyb, self.W[p + "v1"]["wt"], Np, 2 * L, L, EPI_STORE, z=dcat)
             self._k("sphg_gnn_node_concat_bwd", _ptr(dcat), _ptr(dh), _ptr(dagg), b.n, L, s)
-            self._k("sphg_gnn_segsum_bwd", _ptr(dagg), _ptr(b.dst), _ptr(de), b.E, L, AGG_SCALE, s)
             # edge update e' = e + relu(z) W2^T + b2
-            self._bgrad(de, p + "b2", Ep)
-            self._wgrad(de, a, p + "w2", Ep)
-            self._ws(self._bf16(de, "deb"), self.W[p + "w2"]["wt"], Ep, L, L, EPI_STORE, z=da)
-            self._k("sphg_gnn_relu_bwd", _ptr(da), _ptr(z), _ptr(dz), _ptr(dzb), Ep * L, s)
-            self._bgrad(dz, p + "be", Ep)
-            self._wgrad(dz, eb, p + "we", Ep)
+            self._k("sphg_gnn_edge_grad", _ptr(dagg), _ptr(b.dst), _ptr(de), _ptr(deb), _ptr(self.B[p + "b2"]["g"]), b.E,
+                    Ep, AGG_SCALE, 1 if l == LAYERS - 1 and trace is None else 0, s)
+            self._wgrad(deb, a, p + "w2", Ep)
+            self._ws(deb, self.W[p + "w2"]["wt"], Ep, L, L, EPI_RELU_BWD, z=dz, h=dzb, P=z)
+            self._wgrad(dzb, eb, p + "we", Ep)
             self._ws(dzb, self.W[p + "we"]["wt"], Ep, L, L, EPI_ACC, z=de)
             dP.zero_()
             self._k("sphg_gnn_gather_bwd", _ptr(dz), _ptr(b.src), _ptr(b.off), _ptr(dP), b.n, b.E, L, s)
-            self._wgrad(dP, hb, p + "wsd", Np)
-            self._ws(self._bf16(dP, "dPb"), self.W[p + "wsd"]["wt"], Np, L, 2 * L, EPI_ACC, z=dh)
+            # every edge has one receiver: the receiver half of dP sums to the gradient of be
+            dPb = self._cast_bgrad(dP, p + "be", "dPb")
+            self._wgrad(dPb, hb, p + "wsd", Np)
+            self._ws(dPb, self.W[p + "wsd"]["wt"], Np, L, 2 * L, EPI_ACC, z=dh)
         if trace is not None:
             trace["enc"] = (dh.clone(), de.clone())
         # encoders
         for side, d, rows, feat in (("n", dh, Np, b.fn), ("e", de, Ep, b.fe)):
             enc = "enc_" + side
-            zbuf = G(side + "z", (rows, L), f32)
-            abuf = G(side + "a", (rows, L), bf)
-            tmp = G("tmp" + side, (rows, L), f32)
-            self._bgrad(d, enc + ".b2", rows)
-            self._wgrad(d, abuf, enc + ".w2", rows)
-            self._ws(self._bf16(d, "d" + side + "b"), self.W[enc + ".w2"]["wt"], rows, L, L, EPI_STORE, z=tmp)
+            db = self._cast_bgrad(d, enc + ".b2", "d" + side + "b")
+            self._wgrad(db, G(side + "a", (rows, L), bf), enc + ".w2", rows)
             dzz = G("dzz" + side, (rows, L), f32)
-            dzzb = G("dzzb" + side, (rows, L), bf)
-            self._k("sphg_gnn_relu_bwd", _ptr(tmp), _ptr(zbuf), _ptr(dzz), _ptr(dzzb), rows * L, s)
-            self._bgrad(dzz, enc + ".b1", rows)
-            self._wgrad(dzz, feat, enc + ".w1", rows)
+            dzzb = G("dzz" + side + "b", (rows, L), bf)
+            self._ws(db, self.W[enc + ".w2"]["wt"], rows, L, L, EPI_RELU_BWD, z=dzz, h=dzzb, P=G(side + "z", (rows, L), f32))
+            self._cast_bgrad(dzz, enc + ".b1")
+            self._wgrad(dzzb, feat, enc + ".w1", rows)
 
     def adam(self, lr: float, b1=0.9, b2=0.999, eps=1e-8):
         self.adam_step += 1
-        s = self.stream
-        for d in self.W.values():
-            self._k("sphg_gnn_adam", _ptr(d["w"]), _ptr(d["g"]), _ptr(d["m"]), _ptr(d["v"]), _ptr(d["wb"]),
-                    _ptr(d["wt"]), d["rows"], d["cols"], lr, b1, b2, eps, self.adam_step, d["lim"], s)
-        for d in self.B.values():
-            self._k("sphg_gnn_adam", _ptr(d["w"]), _ptr(d["g"]), _ptr(d["m"]), _ptr(d["v"]), None, None,
-                    d["rows"], 1, lr, b1, b2, eps, self.adam_step, d["lim"], s)
+        if self.adam_list is None:
+            ts = list(self.W.values()) + list(self.B.values())
+            self.adam_list = AdamList(len(ts), 0, (AdamTensor * ADAM_MAX)(*[
+                AdamTensor(*(_ptr(d.get(k)) for k in ("w", "g", "m", "v", "wb", "wt")), d["rows"], d.get("cols", 1),
+                           d["lim"], 0) for d in ts]))
+        self._k("sphg_gnn_adam_all", C.addressof(self.adam_list), lr, b1, b2, eps, self.adam_step, self.stream)
 
     def check_device_errors(self):
         if int(self.err.item()) != 0:
