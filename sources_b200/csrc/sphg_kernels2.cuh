@@ -59,7 +59,8 @@ __device__ __forceinline__ float2 inv_rho(float2 rho) {
 // (approaching pairs only), mc = c_a + c_b.
 __device__ __forceinline__ void visc_pair(const PairK& K, float2 rr, float2 dx, float2 dy, float2 du, float2 dv, float2 rho_a,
                                           float rho_b, float m_b, float2 mc, float2& mi, float2& pi) {
-    const float2 mr = add2(rho_a, splat2(rho_b)), den = add2(rr, splat2(K.h2e));
+    // (kept above zero: a particle's own slot and coincident particles have r = 0, and etq may be 0)
+    const float2 mr = add2(rho_a, splat2(rho_b)), de0 = add2(rr, splat2(K.h2e)), den = two(fmaxf(de0.x, 1e-30f), fmaxf(de0.y, 1e-30f));
     const float2 inv = rcp2(mul2(mr, den));
     mi = mul2(mul2(splat2(m_b + m_b), inv), den);
     const float2 vr = fma2(du, dx, mul2(dv, dy));   // -(v_a - v_b) . (x_a - x_b)

@@ -131,3 +131,25 @@ def test_odd_particle_counts(cuda_ok, drop):
         for f, tol in (("x", 5e-7), ("vx", 5e-4), ("rho", 5e-6)):
             x, y = getattr(A, f), getattr(B, f)
             assert np.abs(x - y).max() <= tol * np.abs(x).max(), f
+
+
+@pytest.mark.parametrize("kind", ["granular_column", "two_phase"])
+def test_coincident_particles_without_etq(cuda_ok, kind):
+    """etq = 0 leaves the viscous denominator r^2 alone: a particle's own slot
+    and coincident neighbours (r = 0) add nothing."""
+    s64, s32 = (build(kind, prec, 1, (13, 17, 29), 1.0) for prec in (SPHG_FP64, SPHG_FP32))
+    for s in (s64, s32):
+        s.params.etq = 0.0
+        for P in s.phases:
+            P.x[7] = P.x[6]
+            P.vx[7] = P.vx[6] + 0.05
+    with Solver(s64) as a, Solver(s32) as b:
+        a.single_step(1)
+        b.single_step(1)
+        assert list(a.stats().niac) == list(b.stats().niac)
+        for k, P in enumerate(s64.phases):
+            A, B = a.download(k + 1), b.download(k + 1)
+            for f in ("drho", "dvx", "av"):
+                x, y = getattr(A, f), getattr(B, f)
+                assert np.isfinite(x).all() and np.isfinite(y).all(), f
+                assert np.abs(x - y).max() <= 2e-3 * np.abs(x).max(), f   # the FP32 budget of one step's rates
