@@ -269,8 +269,9 @@ __device__ __forceinline__ int warp_min(int v) {
 // Smoothing kernel with the per-particle constants hoisted out of the pair
 // loop (every pair of a particle shares one h when all h are equal).
 // eval() returns W and the radial factor s with grad W = s * dx, so that
-// dx . grad W = s * r^2.  T = double keeps the IEEE sqrt and divisions of
-// the reference's expression; T = float uses rsqrt/reciprocal.
+// dx . grad W = s * r^2.  r and 1/r come from one rsqrt and q from a product
+// with 1/h (in FP64 too: a sqrt and two divisions per pair, each a serial chain
+// of FP64 operations, were a fifth of the FP64 passes).
 template <typename T> __device__ __forceinline__ T rcp_(T x) { return T(1) / x; }
 template <> __device__ __forceinline__ float rcp_<float>(float x) { return __frcp_rn(x); }
 template <typename T> __device__ __forceinline__ T div_(T a, T b) { return a / b; }
@@ -302,12 +303,14 @@ struct KernelConst {
     // r2 = dx^2 + dy^2 of the pair
     __device__ __forceinline__ void eval(T r2, T& w, T& s) const {
         T r, rinv;
-        if (sizeof(T) == 8) { r = sqrt(r2); rinv = T(1) / r; }
-        else {
+        if (sizeof(T) == 8) {
+            rinv = (T)rsqrt(fmax((double)r2, 1e-300));
+            r = r2 * rinv;
+        } else {
             rinv = (T)rsqrtf((float)fmaxf((float)r2, 1e-30f));
             r = r2 * rinv;
         }
-        const T q = sizeof(T) == 8 ? r / h : r * inv_h;
+        const T q = r * inv_h;
         w = T(0); s = T(0);
         if (SKF == 1) {
             if (q <= T(1)) {

@@ -46,9 +46,8 @@ struct SimConst {
 #ifndef SPHG_X_SPLIT
 #define SPHG_X_SPLIT 4
 #endif
-// minimum resident blocks per SM of each FP32 pair pass (register cap for
-// the compiler: 65,536 / (SPHG_TPB * min blocks) registers per thread); the
-// FP64 passes are left uncapped.  Timed on a B200 at 912,016 particles:
+// minimum resident blocks per SM of each pair pass (register cap for the
+// compiler: 65,536 / (SPHG_TPB * min blocks) registers per thread).  Timed on a B200 at 912,016 particles:
 // water_pass_a (staged, recording the hit masks) 131 us at 8 blocks, 134 at
 // 7, 138 at 10 (48 registers).  water_pass_b (replaying the masks, with the
 // cross pairs) 176 us at 6 blocks, 164 at 7, 181 at 8 (spills).  soil_pass
@@ -71,6 +70,20 @@ struct SimConst {
 #endif
 #ifndef SPHG_MINB_SOIL
 #define SPHG_MINB_SOIL 1
+#endif
+
+// FP64, 912,016 particles: serial chains of FP64 operations, hidden by resident
+// blocks.  water_pass_a 164 us at 4, 5 or 6; water_pass_b 317 uncapped (164
+// registers), 272 at 4, 474 at 5 (spills); soil_pass 139 uncapped (212), 109 at
+// 3, 140 at 4 (spills).
+#ifndef SPHG_MINB_A64
+#define SPHG_MINB_A64 5
+#endif
+#ifndef SPHG_MINB_B64
+#define SPHG_MINB_B64 4
+#endif
+#ifndef SPHG_MINB_S64
+#define SPHG_MINB_S64 3
 #endif
 
 // launch the step's kernels with programmatic stream serialization (0: plain launches)
@@ -478,7 +491,7 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
 // delta_sph's (dx . grad W) 2 (f_a - f_b) / r^2 is evaluated as 2 s (f_a - f_b)
 // since grad W = s dx.
 template <typename T, int SKF, bool SINGLE>
-__global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : 1) k_water_pass_a(PhaseDev<T> P, GridGeom g, SearchConst sc, SimConst c, DevCounters* cnt) {
+__global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : SPHG_MINB_A64) k_water_pass_a(PhaseDev<T> P, GridGeom g, SearchConst sc, SimConst c, DevCounters* cnt) {
     pdl_enter();
     const int k = gtid();
     const bool valid = k < P.n;
@@ -688,7 +701,7 @@ __device__ __forceinline__ void water_b_finish(const PhaseDev<T>& P, const GridG
 // (declarations_sph.f90:1414-1421), then, as the last pass of the water
 // phase, the leapfrog corrector.  FCH as in cross_water_sums.
 template <typename T, int SKF, bool SINGLE, bool FCH>
-__global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : 1) k_water_pass_b(PhaseDev<T> P, PhaseDev<T> S, GridGeom g, SearchConst sc,
+__global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_MINB_B64) k_water_pass_b(PhaseDev<T> P, PhaseDev<T> S, GridGeom g, SearchConst sc,
                                                           SearchConst scx, SimConst c, StepCtl u, DevCounters* cnt) {
     pdl_enter();
     typedef typename V2<T>::t T2;
@@ -741,11 +754,20 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : 1) k_
         d3 = fma2(splat2(vb), mul2(s_b, splat2(gr.y)), d3);
         const T2 dv = sub2(va, vb2);                              // v_a - v_b
         const T mb = vb * rb.rho;
-        const T irho = rcp_<T>(T(0.5) * (ra.rho + rb.rho));       // 1 / mean density (art_visc and av_vel)
+        // 1 / mean density (art_visc and av_vel); in FP64 from one reciprocal with 1 / (r^2 + etq^2 h^2)
+        T irho, iden = T(0);
+        if constexpr (sizeof(T) == 8) {
+            const T mr = T(0.5) * (ra.rho + rb.rho), den = fmax(rr + mh * mh * etq2, T(1e-300));
+            const T inv = T(1) / (mr * den);
+            irho = inv * den;
+            iden = inv * mr;
+        } else {
+            irho = rcp_<T>(T(0.5) * (ra.rho + rb.rho));
+        }
         if (visc) {
             const T vr = dv.x * dx + dv.y * dy;
             if (vr < T(0)) {
-                const T muv = div_<T>(mh * vr, rr + mh * mh * etq2);
+                const T muv = sizeof(T) == 8 ? mh * vr * iden : div_<T>(mh * vr, rr + mh * mh * etq2);
                 const T mc = T(0.5) * (qa.c + qb.c);
                 const T piv = ((beta * muv - alpha * mc) * muv) * irho;
                 av = fma2(splat2(-mb), mul2(splat2(piv), gr), av);
@@ -901,7 +923,7 @@ __device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom
 // last pass of the soil phase, the leapfrog corrector.  FCH as in
 // cross_soil_sums.
 template <typename T, int SKF, bool SINGLE, bool FCH>
-__global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : 1) k_soil_pass(PhaseDev<T> P, PhaseDev<T> W, GridGeom g, SearchConst sc,
+__global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SPHG_MINB_S64) k_soil_pass(PhaseDev<T> P, PhaseDev<T> W, GridGeom g, SearchConst sc,
                                                        SearchConst scx, SimConst c, DevCounters* cnt, int slot, StepCtl u) {
     pdl_enter();
     typedef typename V2<T>::t T2;
@@ -941,6 +963,15 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : 1)
         const T du = rb.vx - ra.vx, dv = rb.vy - ra.vy;   // v_b - v_a
         const T vb = rb.vol, mb = vb * rb.rho;
         const T e = T(2) * sr;                            // 2 (dx . grad W) / r^2
+        // in FP64, 1 / mean density, 1 / (r^2 + etq^2 h^2) and 1 / rho_b from one reciprocal
+        T irho64 = T(0), iden64 = T(0), irb64 = T(0);
+        if constexpr (sizeof(T) == 8) {
+            const T mr = T(0.5) * (ra.rho + rb.rho), den = fmax(rr + mh * mh * etq2, T(1e-300));
+            const T md = mr * den, inv = T(1) / (md * rb.rho);
+            irb64 = inv * md;
+            irho64 = inv * (den * rb.rho);
+            iden64 = inv * (mr * rb.rho);
+        }
         con -= mb * (du * gx + dv * gy);
         if (dens) dl += pref_old * vb * ((ra.rho - rb.rho) * e);
         txx += vb * (c23 * (T(2) * du * gx - dv * gy));
@@ -956,7 +987,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : 1)
             s2y += vb * ((faxy + qb.sxy) * gx);
             s3y += vb * ((fayy + qb.syy) * gy);
         } else {            // df3: m_b (f_a/rho_a^2 + f_b/rho_b^2) gradW
-            const T irb = rcp_<T>(rb.rho);
+            const T irb = sizeof(T) == 8 ? irb64 : rcp_<T>(rb.rho);
             const T ib = qb.vof * irb * irb;
             const T pp = fap * ira2 + qb.p * ib;
             s1x += mb * (pp * gx); s1y += mb * (pp * gy);
@@ -971,9 +1002,10 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : 1)
         if (visc) {
             const T vr = -(du * dx + dv * dy);
             if (vr < T(0)) {
-                const T muv = div_<T>(mh * vr, rr + mh * mh * etq2);
+                const T muv = sizeof(T) == 8 ? mh * vr * iden64 : div_<T>(mh * vr, rr + mh * mh * etq2);
                 const T mrho = T(0.5) * (ra.rho + rb.rho);
-                const T piv = div_<T>((beta * muv - alpha * cs) * muv, mrho);
+                const T pv = (beta * muv - alpha * cs) * muv;
+                const T piv = sizeof(T) == 8 ? pv * irho64 : div_<T>(pv, mrho);
                 avx -= mb * (piv * gx);
                 avy -= mb * (piv * gy);
             }
@@ -994,7 +1026,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : 1)
             }
         }
         if (xsph) {
-            const T q = div_<T>(mb * w, (ra.rho + rb.rho) / T(2));
+            const T q = sizeof(T) == 8 ? mb * w * irho64 : div_<T>(mb * w, (ra.rho + rb.rho) / T(2));
             xsx += q * du;
             xsy += q * dv;
         }
