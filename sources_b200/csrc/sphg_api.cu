@@ -18,6 +18,7 @@
 #include <string>
 #include <system_error>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/sphg.h"
@@ -1147,8 +1148,39 @@ struct Engine : EngineBase {
             if (paired())
                 return launch_pdl("water_pass_a", k_water_pass_a2<SKF>, blocks2(D.n), SPHG_TPB2, Staged2<false>::BYTES, D, grid,
                                   pair_k<SKF>(), sim, cnt);
-        return launch_pdl("water_pass_a", k_water_pass_a<T, SKF, false>, blocks(D.n, SPHG_TPB), SPHG_TPB,
-                          (size_t)SPHG_STAGE_A * (16 + sizeof(RecA<T>)), D, grid, sc_same, sim, cnt);
+        return with_lanes(D.n, [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            return launch_pdl("water_pass_a", k_water_pass_a<T, SKF, false, G>, blocksG(D.n, G), SPHG_TPB,
+                              G == 1 ? (size_t)SPHG_STAGE_A * (16 + sizeof(RecA<T>)) : 0, D, grid, sc_same, sim, cnt);
+        });
+    }
+    // FP64 phases too small to fill the GPU: 8 or 4 lanes per particle
+    // (scan_lanes), since one lane's walk of its candidates is all the time a
+    // pass takes there.  us per step with 1, 4, 8 and 16 lanes, water only: 4.6k
+    // particles 62.5, 43.2, 36.4, 36.5; 8.8k 66.0, 43.0, 39.0, 48.4; 17k 68.4,
+    // 47.2, 54.1; 34k 72.7, 66.2, 79.5; 50k 75.5, 86.5.  Soil only: 4.7k 46.6,
+    // 30.6, 28.1, 34.2; 9k 47.0, 32.3, 36.3; 34k 52.9, 54.9.
+    static int lanes(int n) { return sizeof(T) == 4 || n > 32000 ? 1 : n > 10000 ? 4 : 8; }
+    template <class F>
+    static int with_lanes(int n, F&& f) {   // f(integral_constant G)
+        if constexpr (sizeof(T) == 8) {
+            if (lanes(n) == 8) return f(std::integral_constant<int, 8>());
+            if (lanes(n) == 4) return f(std::integral_constant<int, 4>());
+        }
+        return f(std::integral_constant<int, 1>());
+    }
+    static int blocksG(int n, int g) { return blocks((long long)n * g, SPHG_TPB); }
+    // the passes of the water-only step: 0 density, 1 A, 2 B
+    template <int SKF>
+    int launch_water_only(PhaseDev<T>& D, int pass, const StepCtl& u) {
+        return with_lanes(D.n, [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            const int nb = blocksG(D.n, G);
+            if (pass == 0) return launch_pdl("water_sum", k_water_sum<T, SKF, G>, nb, SPHG_TPB, 0, D, grid, sc_same, sim, cnt);
+            if (pass == 1) return launch_pdl("water_pass_a", k_water_pass_a<T, SKF, true, G>, nb, SPHG_TPB, 0, D, grid, sc_same, sim, cnt);
+            return launch_pdl("water_pass_b", k_water_pass_b<T, SKF, true, false, G>, nb, SPHG_TPB, 0, D, D, grid, sc_same, sc_same,
+                              sim, u, cnt);
+        });
     }
     template <int SKF, bool FCH>
     int launch_water_b(PhaseDev<T>& D, PhaseDev<T>& O, const StepCtl& u) {
@@ -1156,8 +1188,11 @@ struct Engine : EngineBase {
             if (paired())
                 return launch_pdl("water_pass_b", k_water_pass_b2<SKF, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O,
                                   grid, pair_k<SKF>(D.dspp), sim, u, cnt);
-        return launch_pdl("water_pass_b", k_water_pass_b<T, SKF, false, FCH>, blocks(D.n, SPHG_TPB), SPHG_TPB, 0, D, O, grid,
-                          sc_same, sc_cross, sim, u, cnt);
+        return with_lanes(D.n, [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            return launch_pdl("water_pass_b", k_water_pass_b<T, SKF, false, FCH, G>, blocksG(D.n, G), SPHG_TPB, 0, D, O, grid,
+                              sc_same, sc_cross, sim, u, cnt);
+        });
     }
     template <int SKF, bool SINGLE, bool FCH>
     int launch_soil(PhaseDev<T>& D, PhaseDev<T>& O, int slot, const StepCtl& u) {
@@ -1165,14 +1200,16 @@ struct Engine : EngineBase {
             if (paired())
                 return launch_pdl("soil_pass", k_soil_pass2<SKF, SINGLE, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O, grid,
                                   pair_k<SKF>(D.dspp), sim, cnt, slot, u);
-        return launch_pdl("soil_pass", k_soil_pass<T, SKF, SINGLE, FCH>, blocks(D.n, SPHG_TPB), SPHG_TPB, 0, D, O, grid, sc_same,
-                          sc_cross, sim, cnt, slot, u);
+        return with_lanes(D.n, [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            return launch_pdl("soil_pass", k_soil_pass<T, SKF, SINGLE, FCH, G>, blocksG(D.n, G), SPHG_TPB, 0, D, O, grid, sc_same,
+                              sc_cross, sim, cnt, slot, u);
+        });
     }
     template <int SKF>
     int passes(int fh, StepCtl u) {
         const sphg_params& p = ctx->prm;
         u.ncount = nullptr;   // set per phase: the corrector counts that phase's next cells
-        const int tpb = SPHG_TPB;
         const int dp = sim.yield_dp;
         // the paired passes take h from their constants (the water-only step runs the one-particle ones)
         const int hs = paired() && !(p.single_phase && P[0].material == SPHG_WATER) ? 0 : 1;
@@ -1181,12 +1218,11 @@ struct Engine : EngineBase {
             PhaseDev<T>& D = P[0];
             if (D.material == SPHG_WATER) {
                 if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 0, 0, fh, hs, 0, cnt))) return rc;
-                if ((rc = launch_pdl("water_sum", k_water_sum<T, SKF>, blocks(D.n, tpb), tpb, 0, D, grid, sc_same, sim, cnt))) return rc;
-                if ((rc = launch_pdl("water_pass_a", k_water_pass_a<T, SKF, true>, blocks(D.n, tpb), tpb, 0, D, grid, sc_same, sim, cnt))) return rc;
+                if ((rc = launch_water_only<SKF>(D, 0, u))) return rc;
+                if ((rc = launch_water_only<SKF>(D, 1, u))) return rc;
                 StepCtl uw = u;
                 uw.ncount = u.update ? counts[0] : nullptr;
-                if ((rc = launch_pdl("water_pass_b", k_water_pass_b<T, SKF, true, false>, blocks(D.n, tpb), tpb, 0, D, D, grid, sc_same,
-                                 sc_same, sim, uw, cnt))) return rc;
+                if ((rc = launch_water_only<SKF>(D, 2, uw))) return rc;
             } else {
                 if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 1, dp, fh, hs, dp, cnt))) return rc;
                 StepCtl us = u; us.with_vof = 0; us.do_dp = dp;

@@ -528,6 +528,39 @@ __device__ __forceinline__ int scan_direct(const SearchConst& sc, const CandRuns
     return hits;
 }
 
+// The same visit by G neighbouring lanes, each testing every G-th candidate of
+// one particle: for grids too small to fill the GPU, whose passes take as long
+// as one lane's serial walk of its candidates.  The lanes' sums are added with
+// lanes_sum; hits is this lane's share.
+template <int G, typename T, class F>
+__device__ __forceinline__ int scan_lanes(const SearchConst& sc, const CandRuns& cr, const double2* __restrict__ xs,
+                                          const double* __restrict__ hs, double2 xa, double ha, int self, F&& body) {
+    int hits = 0;
+    const int tot = cr.total();
+    for (int t = threadIdx.x % G; t < tot; t += G) {
+        const int m = cr.at(t);
+        if (m == self) continue;
+        const double2 xb = xs[m];
+        const double dx = xa.x - xb.x, dy = xa.y - xb.y;
+        const double r2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+        if (sc.uniform ? (r2 < sc.r2_uniform) : (__dsqrt_rn(r2) < sc.scale_k * ((ha + hs[m]) / 2.0))) {
+            ++hits;
+            body(m, (T)dx, (T)dy);
+        }
+    }
+    return hits;
+}
+template <int G, typename T>
+__device__ __forceinline__ void lanes_sum(T& v) {
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+}
+template <int G, typename T, typename... R>
+__device__ __forceinline__ void lanes_sum(T& v, R&... rest) {
+    lanes_sum<G>(v);
+    lanes_sum<G>(rest...);
+}
+
 // The same visit replayed from the hit mask an earlier pass of this step
 // recorded over the same sorted positions: the same neighbours in the same
 // order, so every sum is bit-identical, without testing any candidate again.

@@ -337,6 +337,8 @@ __device__ __forceinline__ void count_stats(DevCounters* cnt, int list, int phas
 // support 2h = 2.4 dx in one drain (FP32); FP64 entries are larger.
 template <typename T> struct Chunk { static const int value = sizeof(T) == 4 ? 24 : 16; };
 #define SPHG_HITBUF(T) __shared__ HitBuf<T, SPHG_TPB, Chunk<T>::value> hb
+// (one entry when the pass does not use it)
+#define SPHG_HITBUF_G(T, G) __shared__ HitBuf<T, (G) == 1 ? SPHG_TPB : 1, (G) == 1 ? Chunk<T>::value : 1> hb
 
 // Kernel constants for particle a: per particle when every h is equal, else
 // per pair (mhsml = (h_a + h_b)/2).
@@ -376,11 +378,11 @@ __device__ __forceinline__ void water_sum_finish(const PhaseDev<T>& P, const Sim
     P.countiac[a] = hits;
 }
 
-template <typename T, int SKF>
+// G > 1: G lanes per particle (scan_lanes), no hit masks.
+template <typename T, int SKF, int G = 1>
 __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom g, SearchConst sc, SimConst c, DevCounters* cnt) {
     pdl_enter();
-    SPHG_HITBUF(T);
-    const int k = gtid();
+    const int k = gtid() / G;
     const bool valid = k < P.n;
     const int kk = valid ? k : 0;
     const double2 xa = P.xs[kk];
@@ -396,7 +398,7 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
     T sx = T(0), sy = T(0);
     const RecA<T>* __restrict__ rec = P.recA;
     uint4 mask;
-    const int hits = visit_batched_rec(hb, g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, mask, [&](int m, T dx, T dy) {
+    auto body = [&](int m, T dx, T dy) {
         const RecA<T> rb = rec[m];
         T w, sr, r2, mh;
         pair_kernel<T, SKF>(ka, sc, ha, P.hs, m, dx, dy, w, sr, r2, mh);
@@ -405,12 +407,21 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
         num += mb * w;
         sx += mb * ((rb.vx - ra.vx) * (sr * dx));
         sy += mb * ((rb.vy - ra.vy) * (sr * dy));
-    });
-    if (valid) {
-        if (P.hmask) P.hmask[k] = mask;
-        water_sum_finish(P, c, k, ra, num, wi, sx, sy, hits);
+    };
+    int hits;
+    bool finish = valid;
+    if constexpr (G == 1) {
+        SPHG_HITBUF(T);
+        hits = visit_batched_rec(hb, g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, mask, body);
+        if (valid && P.hmask) P.hmask[k] = mask;
+    } else {
+        finish = valid && threadIdx.x % G == 0;
+        if (threadIdx.x % G) { wi = T(0); num = T(0); }
+        hits = scan_lanes<G, T>(sc, candidate_runs(g, P.cell_start, xa, valid), P.xs, P.hs, xa, ha, k, body);
+        lanes_sum<G>(wi, num, sx, sy, hits);
     }
-    count_stats(cnt, 0, 0, hits, valid);
+    if (finish) water_sum_finish(P, c, k, ra, num, wi, sx, sy, hits);
+    count_stats(cnt, 0, 0, hits, finish);
 }
 
 // r^3 to within rounding: the product and the rounding errors of its factors.
@@ -490,10 +501,11 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
 //   delta_sph on the summation density, Tait without vof, t = df(v) form.
 // delta_sph's (dx . grad W) 2 (f_a - f_b) / r^2 is evaluated as 2 s (f_a - f_b)
 // since grad W = s dx.
-template <typename T, int SKF, bool SINGLE>
+// G as in k_water_sum.
+template <typename T, int SKF, bool SINGLE, int G = 1>
 __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : SPHG_MINB_A64) k_water_pass_a(PhaseDev<T> P, GridGeom g, SearchConst sc, SimConst c, DevCounters* cnt) {
     pdl_enter();
-    const int k = gtid();
+    const int k = gtid() / G;
     const bool valid = k < P.n;
     const int kk = valid ? k : 0;
     const int a = P.perm[kk];
@@ -508,7 +520,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : SPHG_
     ka.init((T)ha);
     T con = 0, dl = 0, t0 = 0, t1 = 0, t2 = 0, t3 = 0;
     uint4 mask = make_uint4(0u, 0u, 0u, 0u);
-    if (SINGLE && valid) mask = P.hmask[k];   // recorded by k_water_sum
+    if (SINGLE && G == 1 && valid) mask = P.hmask[k];   // recorded by k_water_sum
     auto body = [&](const RecA<T>* R, int m, T dx, T dy) {
         const RecA<T> rb = R[m];
         T w, sr, r2, mh;
@@ -530,7 +542,13 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : SPHG_
         }
     };
     int hits;
-    if constexpr (SINGLE) {
+    bool finish = valid;
+    if constexpr (G > 1) {
+        finish = valid && threadIdx.x % G == 0;
+        hits = scan_lanes<G, T>(sc, candidate_runs(g, P.cell_start, xa, valid), P.xs, P.hs, xa, ha, k,
+                                [&](int m, T dx, T dy) { body(rec, m, dx, dy); });
+        lanes_sum<G>(con, dl, t0, t1, t2, t3, hits);
+    } else if constexpr (SINGLE) {
         hits = visit_masked<T>(g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, mask,
                                [&](int m, T dx, T dy) { body(rec, m, dx, dy); });
     } else {
@@ -558,11 +576,11 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : SPHG_
                                         [&](int m, T dx, T dy) { body(rec, m, dx, dy); });
         }
     }
-    if (valid) {
-        if (!SINGLE) P.hmask[k] = mask;
+    if (finish) {
+        if (!SINGLE && G == 1) P.hmask[k] = mask;
         water_a_finish<T, SINGLE>(P, c, k, con, dl, t0, t1, t2, t3, hits);
     }
-    if (!SINGLE) count_stats(cnt, 0, 0, hits, valid);
+    if (!SINGLE) count_stats(cnt, 0, 0, hits, finish);
 }
 
 // ------------------------------------------------------------- cross phase
@@ -577,11 +595,11 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_A : SPHG_
 // vol_w*rho_w*vof_w*vof_s*(-g/k)*(v_w - v_s)*W/rho_s; the sums here are the
 // pair parts, the particle factors are applied by the caller.  The pore
 // pressure m_w p_w/(rho_w rho_s) becomes vol_w p_w / rho_s.
-template <typename T, int SKF, bool FCH, class HB>
-__device__ __forceinline__ void cross_soil_sums(HB& hb, const PhaseDev<T>& W, const GridGeom& g, const SearchConst& sc,
-                                                const SimConst& c, const KernelConst<T, SKF>& ka, double2 xa, double ha,
-                                                const RecA<T>& ra, bool valid, T& ddx, T& ddy, T& dpx, T& dpy) {
-    visit_batched(hb, g, sc, W.cell_start, W.xs, W.hs, xa, ha, -1, valid, [&](int m, T dx, T dy) {
+template <typename T, int SKF, bool FCH, class V>
+__device__ __forceinline__ void cross_soil_sums(V&& visit, const PhaseDev<T>& W, const SearchConst& sc,
+                                                const SimConst& c, const KernelConst<T, SKF>& ka, double ha,
+                                                const RecA<T>& ra, T& ddx, T& ddy, T& dpx, T& dpy) {
+    visit([&](int m, T dx, T dy) {
         const RecA<T> rb = W.recA[m];
         const RecB<T> qb = W.recB[m];
         T w, sr, rr, mh;
@@ -601,11 +619,11 @@ __device__ __forceinline__ void cross_soil_sums(HB& hb, const PhaseDev<T>& W, co
 
 // Water side: darcy_law :3832, volume_fraction_water2 :3940 (dvof) and
 // volume_fraction_water :3912 (vof2).  Returns the number of pairs.
-template <typename T, int SKF, bool FCH, class HB>
-__device__ __forceinline__ int cross_water_sums(HB& hb, const PhaseDev<T>& S, const GridGeom& g, const SearchConst& sc,
-                                                const SimConst& c, const KernelConst<T, SKF>& ka, double2 xa, double ha,
-                                                const RecA<T>& ra, bool valid, T& ddx, T& ddy, T& dvof, T& v2) {
-    return visit_batched(hb, g, sc, S.cell_start, S.xs, S.hs, xa, ha, -1, valid, [&](int m, T dx, T dy) {
+template <typename T, int SKF, bool FCH, class V>
+__device__ __forceinline__ int cross_water_sums(V&& visit, const PhaseDev<T>& S, const SearchConst& sc,
+                                                const SimConst& c, const KernelConst<T, SKF>& ka, double ha,
+                                                const RecA<T>& ra, T& ddx, T& ddy, T& dvof, T& v2) {
+    return visit([&](int m, T dx, T dy) {
         const RecA<T> rb = S.recA[m];
         const T phis = S.recB[m].vof;
         T w, sr, rr, mh;
@@ -700,13 +718,12 @@ __device__ __forceinline__ void water_b_finish(const PhaseDev<T>& P, const GridG
 // rho/vof*vof2, vof <- vof2 every renorm_interval steps
 // (declarations_sph.f90:1414-1421), then, as the last pass of the water
 // phase, the leapfrog corrector.  FCH as in cross_water_sums.
-template <typename T, int SKF, bool SINGLE, bool FCH>
+template <typename T, int SKF, bool SINGLE, bool FCH, int G = 1>
 __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_MINB_B64) k_water_pass_b(PhaseDev<T> P, PhaseDev<T> S, GridGeom g, SearchConst sc,
                                                           SearchConst scx, SimConst c, StepCtl u, DevCounters* cnt) {
     pdl_enter();
     typedef typename V2<T>::t T2;
-    SPHG_HITBUF(T);
-    const int k = gtid();
+    const int k = gtid() / G;
     const bool valid = k < P.n;
     const int kk = valid ? k : 0;
     const int a = P.perm[kk];
@@ -733,7 +750,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
     T2 fa_a, fa_b, va;
     fa_a.x = fa_xx; fa_a.y = fa_xy; fa_b.x = fa_xy; fa_b.y = fa_yy;
     va.x = ra.vx; va.y = ra.vy;
-    const uint4 mask = valid ? P.hmask[k] : make_uint4(0u, 0u, 0u, 0u);   // recorded by the step's first water pass
+    const uint4 mask = G == 1 && valid ? P.hmask[k] : make_uint4(0u, 0u, 0u, 0u);   // recorded by the step's first water pass
     auto body = [&](const RecA<T>* RA, const RecB<T>* RB, int m, T dx, T dy) {
         const RecA<T> rb = RA[m];
         const RecB<T> qb = RB[m];
@@ -792,8 +809,13 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
     // against 164 us for this form at 7 blocks.  Loading each lane's next
     // hit's records during the current one (16 more registers) measured 210
     // us at 6 blocks.
-    visit_masked<T>(g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, mask,
-                    [&](int m, T dx, T dy) { body(rec, P.recB, m, dx, dy); });
+    auto each = [&](int m, T dx, T dy) { body(rec, P.recB, m, dx, dy); };
+    if constexpr (G == 1) {
+        visit_masked<T>(g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, mask, each);
+    } else {
+        scan_lanes<G, T>(sc, candidate_runs(g, P.cell_start, xa, valid), P.xs, P.hs, xa, ha, k, each);
+        lanes_sum<G>(d1.x, d1.y, d2.x, d2.y, d3.x, d3.y, av.x, av.y, rp.x, rp.y, xv.x, xv.y, dvf);
+    }
     const T d1x = d1.x, d1y = d1.y, d2x = d2.x, d2y = d2.y, d3x = d3.x, d3y = d3.y;
     const T avx = av.x, avy = av.y, rpx = rp.x, rpy = rp.y, xsx = xv.x, xsy = xv.y;
     WaterB<T> w;
@@ -804,10 +826,18 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
     w.dvf = dvf;
     w.cdx = w.cdy = w.cdvof = w.cv2 = T(0);
     w.chits = 0;
-    if constexpr (!SINGLE)
-        w.chits = cross_water_sums<T, SKF, FCH>(hb, S, g, scx, c, ka, xa, ha, ra, valid, w.cdx, w.cdy, w.cdvof, w.cv2);
-    if (valid) water_b_finish<T, SINGLE>(P, g, c, u, cnt, k, ra.rho, phia, w);
-    if constexpr (!SINGLE) count_stats(cnt, 2, -1, w.chits, valid);
+    const bool finish = valid && threadIdx.x % G == 0;
+    if constexpr (!SINGLE && G == 1) {
+        SPHG_HITBUF(T);
+        w.chits = cross_water_sums<T, SKF, FCH>([&](auto&& f) { return visit_batched(hb, g, scx, S.cell_start, S.xs, S.hs, xa, ha, -1, valid, f); },
+                                                S, scx, c, ka, ha, ra, w.cdx, w.cdy, w.cdvof, w.cv2);
+    } else if constexpr (!SINGLE) {
+        w.chits = cross_water_sums<T, SKF, FCH>([&](auto&& f) { return scan_lanes<G, T>(scx, candidate_runs(g, S.cell_start, xa, valid), S.xs, S.hs, xa, ha, -1, f); },
+                                                S, scx, c, ka, ha, ra, w.cdx, w.cdy, w.cdvof, w.cv2);
+        lanes_sum<G>(w.cdx, w.cdy, w.cdvof, w.cv2, w.chits);
+    }
+    if (finish) water_b_finish<T, SINGLE>(P, g, c, u, cnt, k, ra.rho, phia, w);
+    if constexpr (!SINGLE) count_stats(cnt, 2, -1, w.chits, finish);
 }
 
 // A soil particle's sums of soil_pass: momentum (before the division by rho),
@@ -922,13 +952,11 @@ __device__ __forceinline__ void soil_finish(const PhaseDev<T>& P, const GridGeom
 // same kernel (cross_soil_sums), then volume_fraction_soil :3970 and, as the
 // last pass of the soil phase, the leapfrog corrector.  FCH as in
 // cross_soil_sums.
-template <typename T, int SKF, bool SINGLE, bool FCH>
+template <typename T, int SKF, bool SINGLE, bool FCH, int G = 1>
 __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SPHG_MINB_S64) k_soil_pass(PhaseDev<T> P, PhaseDev<T> W, GridGeom g, SearchConst sc,
                                                        SearchConst scx, SimConst c, DevCounters* cnt, int slot, StepCtl u) {
     pdl_enter();
-    typedef typename V2<T>::t T2;
-    SPHG_HITBUF(T);
-    const int k = gtid();
+    const int k = gtid() / G;
     const bool valid = k < P.n;
     const int kk = valid ? k : 0;
     const int a = P.perm[kk];
@@ -954,7 +982,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
     T s1x = 0, s1y = 0, s2x = 0, s3x = 0, s2y = 0, s3y = 0;
     T avx = 0, avy = 0, rpx = 0, rpy = 0, xsx = 0, xsy = 0;
     T dpp = 0, dsx = 0, dsxy = 0, dsy = 0;
-    const int hits = visit_batched(hb, g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, [&](int m, T dx, T dy) {
+    auto body = [&](int m, T dx, T dy) {
         const RecA<T> rb = P.recA[m];
         const RecB<T> qb = P.recB[m];
         T w, sr, rr, mh;
@@ -1030,7 +1058,17 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
             xsx += q * du;
             xsy += q * dv;
         }
-    });
+    };
+    int hits;
+    const bool finish = valid && threadIdx.x % G == 0;
+    SPHG_HITBUF_G(T, G);
+    if constexpr (G == 1) {
+        hits = visit_batched(hb, g, sc, P.cell_start, P.xs, P.hs, xa, ha, k, valid, body);
+    } else {
+        hits = scan_lanes<G, T>(sc, candidate_runs(g, P.cell_start, xa, valid), P.xs, P.hs, xa, ha, k, body);
+        lanes_sum<G>(con, dl, txx, txy, tyy, vcc, wxy, s1x, s1y, s2x, s3x, s2y, s3y);
+        lanes_sum<G>(avx, avy, rpx, rpy, xsx, xsy, dpp, dsx, dsxy, dsy, hits);
+    }
     SoilSums<T> w;
     if (SINGLE) { w.mx = -s1x + s2x + s3x; w.my = -s1y + s2y + s3y; }
     else {
@@ -1044,11 +1082,17 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
     w.dp = dpp; w.dsx = dsx; w.dsxy = dsxy; w.dsy = dsy;
     w.cdx = w.cdy = w.cpx = w.cpy = T(0);
     w.hits = hits;
-    if constexpr (!SINGLE)
-        cross_soil_sums<T, SKF, FCH>(hb, W, g, scx, c, ka, xa, ha, ra, valid, w.cdx, w.cdy, w.cpx, w.cpy);
+    if constexpr (!SINGLE && G == 1) {
+        cross_soil_sums<T, SKF, FCH>([&](auto&& f) { return visit_batched(hb, g, scx, W.cell_start, W.xs, W.hs, xa, ha, -1, valid, f); },
+                                     W, scx, c, ka, ha, ra, w.cdx, w.cdy, w.cpx, w.cpy);
+    } else if constexpr (!SINGLE) {
+        cross_soil_sums<T, SKF, FCH>([&](auto&& f) { return scan_lanes<G, T>(scx, candidate_runs(g, W.cell_start, xa, valid), W.xs, W.hs, xa, ha, -1, f); },
+                                     W, scx, c, ka, ha, ra, w.cdx, w.cdy, w.cpx, w.cpy);
+        lanes_sum<G>(w.cdx, w.cdy, w.cpx, w.cpy);
+    }
     int fail = 0, fail3 = 0;
-    if (valid) soil_finish<T, SINGLE>(P, g, c, u, cnt, k, ra.rho, qa.vof, w, fail, fail3);
-    count_stats(cnt, slot, slot, hits, valid);
+    if (finish) soil_finish<T, SINGLE>(P, g, c, u, cnt, k, ra.rho, qa.vof, w, fail, fail3);
+    count_stats(cnt, slot, slot, hits, finish);
     if (c.plasticity == 3) count_fail(cnt, 2, fail);
     if (u.update && u.do_dp) count_fail(cnt, 3, fail3);
 }
