@@ -5,7 +5,6 @@
 // float for SPHG_FP32).  One context owns one CUDA stream; every launch and
 // copy goes to that stream (or to a stream the caller sets).
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -299,9 +298,8 @@ struct Engine : EngineBase {
     int ncell = 0;
     int* counts[2] = {nullptr, nullptr};
     int* cell_start_buf[2] = {nullptr, nullptr};
-    void* cub_tmp = nullptr;
-    void* cub_tmp1 = nullptr;        // the second phase's scan, which may run beside the first's
-    size_t cub_bytes = 0;
+    int* chunk_sums[2] = {nullptr, nullptr};     // of k_cell_sums, per phase (the phases' scans may run side by side)
+    int* scattered[2] = {nullptr, nullptr};      // the cell list before its cells are ordered (k_gather)
     // The step's counters and the sticky flags side by side on the device.
     // Each step's check also writes them into mapped pinned host memory
     // (hblk), which the host reads after a batch with no copy; without it
@@ -545,6 +543,8 @@ struct Engine : EngineBase {
                        D.dvof, D.dsxx, D.dsxy, D.dsyy, D.dp, D.txx, D.txy, D.tyy, D.vcc, D.wxy, D.vof2, D.dv, D.av,
                        D.countiac, D.cell_id, D.cell_fill, D.perm, D.xs, D.hs, D.recA, D.recA2, D.recB, D.hmask};
         for (void* p : old) release(p);
+        release(scattered[ph]);
+        scattered[ph] = nullptr;
         for (void* p : shadow[ph]) release(p);
         shadow[ph].clear();
         par[ph] = 0;
@@ -564,6 +564,7 @@ struct Engine : EngineBase {
         rc |= alloc(&D.tyy, N); rc |= alloc(&D.vcc, N); rc |= alloc(&D.wxy, N); rc |= alloc(&D.vof2, N);
         rc |= alloc(&D.dv, N); rc |= alloc(&D.av, N);
         rc |= alloc(&D.countiac, N); rc |= alloc(&D.cell_id, N); rc |= alloc(&D.cell_fill, N); rc |= alloc(&D.perm, N);
+        rc |= alloc(&scattered[ph], N);
         rc |= alloc(&D.xs, N); rc |= alloc(&D.hs, N);
         rc |= alloc(&D.recA, N); rc |= alloc(&D.recA2, N); rc |= alloc(&D.recB, N); rc |= alloc(&D.hmask, N);
         if (rc) return SPHG_ERR_CUDA;
@@ -939,8 +940,7 @@ struct Engine : EngineBase {
                 release(counts[ph]); counts[ph] = nullptr;
                 release(cell_start_buf[ph]); cell_start_buf[ph] = nullptr;
             }
-            release(cub_tmp); cub_tmp = nullptr;
-            release(cub_tmp1); cub_tmp1 = nullptr;
+            for (int ph = 0; ph < 2; ++ph) { release(chunk_sums[ph]); chunk_sums[ph] = nullptr; }
             ncell = nc;
         }
         for (int ph = 0; ph < ctx->nphase; ++ph) {
@@ -948,15 +948,8 @@ struct Engine : EngineBase {
             if (!cell_start_buf[ph] && alloc(&cell_start_buf[ph], (size_t)nc + 1)) return SPHG_ERR_CUDA;
             P[ph].cell_start = cell_start_buf[ph];
         }
-        if (!cub_tmp) {
-            size_t bytes = 0;
-            cub::DeviceScan::ExclusiveSum(nullptr, bytes, counts[0], P[0].cell_start, nc + 1, ctx->stream);
-            size_t b2 = 0;
-            cub::DeviceScan::ExclusiveSum(nullptr, b2, (long long*)nullptr, (long long*)nullptr, nmax + 1, ctx->stream);
-            cub_bytes = std::max(bytes, b2);
-            if (alloc((char**)&cub_tmp, cub_bytes)) return SPHG_ERR_CUDA;
-        }
-        if (ctx->nphase == 2 && !cub_tmp1 && alloc((char**)&cub_tmp1, cub_bytes)) return SPHG_ERR_CUDA;
+        for (int ph = 0; ph < ctx->nphase; ++ph)
+            if (!chunk_sums[ph] && alloc(&chunk_sums[ph], (size_t)blocks(nc, kScanChunk))) return SPHG_ERR_CUDA;
         for (int ph = 0; state_order == 1 && ph < ctx->nphase; ++ph) {   // outside any stream capture
             MortonScratch& M = morton[ph];
             const int n = P[ph].n;
@@ -988,7 +981,7 @@ struct Engine : EngineBase {
         // spatial order from the start
         cells_ready = false;
         for (int ph = 0; ph < ctx->nphase; ++ph) {
-            int rc = build_cells(ph);
+            int rc = build_cells(ph, true);
             if (rc) return rc;
             if ((rc = reorder(ph))) return rc;
         }
@@ -1007,27 +1000,42 @@ struct Engine : EngineBase {
     // Count the current positions' cells as a corrector would have, so that a
     // captured step (which expects them) can run.
     int prime_cells() {
-        if (cells_ready) return 0;
-        for (int ph = 0; ph < ctx->nphase; ++ph) {
-            int rc = count_cells(ph, 1);
+        if (!cells_ready) {
+            // clamped and non-finite positions of the new count only
+            int rc = launch_pdl("reset", k_reset_counters, 1, 32, 0, cnt, 0);
+            for (int ph = 0; !rc && ph < ctx->nphase; ++ph) rc = count_cells(ph, 1);
             if (rc) return rc;
+            cells_ready = true;
+            counters_ready = false;
         }
-        cells_ready = true;
+        if (!counters_ready && hblk) {
+            int rc = launch_pdl("reset", k_reset_counters, 1, 32, 0, cnt, 1);
+            if (rc) return rc;
+            counters_ready = true;
+        }
         return 0;
     }
-    int build_cells(int ph) {
+    // The cell list of a phase, its cells in order (sorted), or left for the
+    // gather to order (then in scattered[ph]).
+    int build_cells(int ph, bool sorted) {
         PhaseDev<T>& D = P[ph];
         int rc = 0;
         if (!cells_ready && (rc = count_cells(ph, 0))) return rc;
-        size_t bytes = cub_bytes;
-        CUDA_TRY(cub::DeviceScan::ExclusiveSum(ph == 1 && cub_tmp1 ? cub_tmp1 : cub_tmp, bytes, counts[ph], D.cell_start,
-                                               ncell + 1, ctx->stream));
-        if ((rc = launch_pdl("cell_scatter", k_cell_scatter, blocks(D.n, 256), 256, 0, D.n, (const int*)D.cell_id,
-                             (const int*)D.cell_fill, (const int*)D.cell_start, D.perm)))
+        const int chunks = blocks(ncell, kScanChunk);
+        const int* sums = ncell > kScanDirect ? chunk_sums[ph] : nullptr;
+        if (sums && (rc = launch_pdl("cell_sums", k_cell_sums, chunks, 256, 0, (const int*)counts[ph], ncell, chunk_sums[ph])))
             return rc;
+        if ((rc = launch_pdl("cell_scan", k_cell_scan, chunks, 256, 0, (const int*)counts[ph], ncell, D.cell_start, sums))) return rc;
+        if ((rc = launch_pdl("cell_scatter", k_cell_scatter, blocks(D.n, 256), 256, 0, D.n, (const int*)D.cell_id,
+                             (const int*)D.cell_fill, (const int*)D.cell_start, sorted ? D.perm : scattered[ph], counts[ph], ncell)))
+            return rc;
+        if (!sorted) return 0;
         return launch_pdl("cell_sort", k_cell_sort, blocks(ncell, 256), 256, 0, ncell, (const int*)D.cell_start,
-                          (const int*)D.orig, D.perm, counts[ph]);
+                          (const int*)D.orig, D.perm);
     }
+    // what the gather of a step reads: the unordered cell list, or null when it was sorted for a reorder
+    const int* unsorted(int ph) const { return reorder_step ? nullptr : scattered[ph]; }
+    bool reorder_step = false;
 
     // The persistent per-particle fields of a phase and their element sizes.
     std::vector<std::pair<void**, int>> field_refs(int ph) {
@@ -1106,7 +1114,13 @@ struct Engine : EngineBase {
     }
 
     // -------------------------------------------------------------- the step
-    int reset_counters() { return launch_pdl("reset", k_reset_counters, 1, 32, 0, cnt, cells_ready ? 1 : 0); }
+    // The counters at a step's start: reset by the last step's check (then its
+    // corrector has counted the cells), else here.
+    bool counters_ready = false;
+    int reset_counters() {
+        if (cells_ready && counters_ready) return 0;
+        return launch_pdl("reset", k_reset_counters, 1, 32, 0, cnt, cells_ready ? 1 : 0);
+    }
 
     // The pair passes of one step for kernel function SKF.  fh: run the
     // leapfrog predictor inside the gathers; u: what the last pass of each
@@ -1217,14 +1231,14 @@ struct Engine : EngineBase {
         if (p.single_phase) {
             PhaseDev<T>& D = P[0];
             if (D.material == SPHG_WATER) {
-                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 0, 0, fh, hs, 0, cnt))) return rc;
+                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 0, 0, fh, hs, 0, cnt, unsorted(0)))) return rc;
                 if ((rc = launch_water_only<SKF>(D, 0, u))) return rc;
                 if ((rc = launch_water_only<SKF>(D, 1, u))) return rc;
                 StepCtl uw = u;
                 uw.ncount = u.update ? counts[0] : nullptr;
                 if ((rc = launch_water_only<SKF>(D, 2, uw))) return rc;
             } else {
-                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 1, dp, fh, hs, dp, cnt))) return rc;
+                if ((rc = launch_pdl("gather", k_gather<T>, blocks(D.n, 256), 256, 0, D, sim, 1, dp, fh, hs, dp, cnt, unsorted(0)))) return rc;
                 StepCtl us = u; us.with_vof = 0; us.do_dp = dp;
                 us.ncount = u.update ? counts[0] : nullptr;
                 if ((rc = launch_soil<SKF, true, false>(D, D, 0, us))) return rc;
@@ -1237,7 +1251,7 @@ struct Engine : EngineBase {
             uw.ncount = u.update ? counts[0] : nullptr;
             us.ncount = u.update ? counts[1] : nullptr;
             // the soil's gather was launched by run() on the side stream
-            if ((rc = launch_pdl("gather", k_gather<T>, blocks(W.n, 256), 256, 0, W, sim, 0, 0, fh, hs, 0, cnt))) return rc;
+            if ((rc = launch_pdl("gather", k_gather<T>, blocks(W.n, 256), 256, 0, W, sim, 0, 0, fh, hs, 0, cnt, unsorted(0)))) return rc;
             if ((rc = launch_water_a<SKF>(W))) return rc;
             // The cross pairs run inside the last pass of each phase; the soil
             // pass reads the water pressure that water_pass_a sets.  After
@@ -1386,6 +1400,7 @@ struct Engine : EngineBase {
         if ((rc = reset_counters())) return rc;
         const sphg_params& p = ctx->prm;
         bool reorder_now = p.reorder_interval > 0 && itimestep > 0 && itimestep % p.reorder_interval == 0;
+        reorder_step = reorder_now;
         if (ctx->nphase == 2 && !p.single_phase) {
             // The soil's cell list, reorder and gather touch soil data only,
             // so they run on the side stream beside the water's (serially
@@ -1398,21 +1413,21 @@ struct Engine : EngineBase {
                 CUDA_TRY(cudaStreamWaitEvent(side, ctx->ev_fork2, 0));
             }
             ctx->stream = side;
-            rc = build_cells(1);
+            rc = build_cells(1, reorder_now);
             if (!rc && reorder_now) rc = reorder(1);
             if (!rc) rc = launch_pdl("gather", k_gather<T>, blocks(P[1].n, 256), 256, 0, P[1], sim, 1, sim.yield_dp, fh,
-                                 paired() ? 0 : 1, sim.yield_dp, cnt);
+                                 paired() ? 0 : 1, sim.yield_dp, cnt, unsorted(1));
             cudaError_t ej = side != main_stream ? cudaEventRecord(ctx->ev_join2, side) : cudaSuccess;
             ctx->stream = main_stream;
             if (rc || ej != cudaSuccess) {
                 if (side != main_stream && ej == cudaSuccess) cudaStreamWaitEvent(main_stream, ctx->ev_join2, 0);
                 return rc ? rc : SPHG_ERR_CUDA;
             }
-            if ((rc = build_cells(0))) return rc;
+            if ((rc = build_cells(0, reorder_now))) return rc;
             if (reorder_now && (rc = reorder(0))) return rc;
         } else {
             for (int ph = 0; ph < ctx->nphase; ++ph) {
-                if ((rc = build_cells(ph))) return rc;
+                if ((rc = build_cells(ph, reorder_now))) return rc;
                 if (reorder_now && (rc = reorder(ph))) return rc;
             }
         }
@@ -1425,8 +1440,9 @@ struct Engine : EngineBase {
         // a step with the corrector has counted the next step's cells
         cells_ready = rc == 0 && u.update != 0;
         if (rc) return rc;
-        return launch_pdl("check", k_check, 1, 32, 0, (const DevCounters*)cnt, sticky, (unsigned long long)p.max_interaction,
-                          hblk_dev);
+        counters_ready = cells_ready && hblk_dev != nullptr;
+        return launch_pdl("check", k_check, 1, 32, 0, cnt, sticky, (unsigned long long)p.max_interaction, hblk_dev,
+                          counters_ready ? 1 : 0);
     }
 
     // single_step / single_step_for_water / single_step_for_soil
@@ -1566,8 +1582,8 @@ struct Engine : EngineBase {
         // the lists of the current positions (the last step's pair search if no
         // step ran since): rebuild sorted positions for both phases
         for (int ph = 0; ph < ctx->nphase; ++ph) {
-            if ((rc = build_cells(ph))) { cells_ready = false; return rc; }
-            if ((rc = launch("gather", k_gather<T>, blocks(P[ph].n, 256), 256, P[ph], sim, 0, 0, 0, 1, 0, cnt))) {
+            if ((rc = build_cells(ph, true))) { cells_ready = false; return rc; }
+            if ((rc = launch("gather", k_gather<T>, blocks(P[ph].n, 256), 256, P[ph], sim, 0, 0, 0, 1, 0, cnt, (const int*)nullptr))) {
                 cells_ready = false;
                 return rc;
             }

@@ -4,7 +4,7 @@
 //   k_first_half      leapfrog predictor (+ Drucker-Prager on soil)      elementwise
 //   k_cell_count      cell key per particle, rank inside its cell         elementwise
 //   k_cell_scatter    counting-sort scatter into cell order              elementwise
-//   k_cell_sort       order each cell by state index (determinism)       per cell
+//   k_cell_sort       order each cell by original index (reorder steps; else in the gather)  per cell
 //   k_gather          sorted copies: x, h, (v, m, rho); soil: DP + stress pair pass inputs
 //   k_water_sum       summation density (water-only step)                pair pass
 //   k_water_pass_a    continuity / df2, delta-SPH(rho), strain rate, EOS  pair pass
@@ -127,32 +127,132 @@ static __global__ void __launch_bounds__(256) k_cell_count(const double2* __rest
     cell_key(g, x[a], a, cell_id, rank, counts, cnt, next);
 }
 
+// Exclusive scan of the cells' counts, start[ncell] = the total: each block
+// scans a chunk of kScanChunk counts on top of the sum of all counts before it,
+// taken from the chunk sums of k_cell_sums or, for few cells, from the counts
+// themselves (one launch instead of two below 64k cells).  Bound: launches and
+// their latency.  With the cells ordered inside the gather and the counters
+// reset by the step's check, us per step before and after: 7.4k particles 33.4,
+// 28.4; 150k 95, 91; 190k 77, 70; 330k 172, 165; 912k 325, 316; the ensemble's
+// dry group 121, 104.
+constexpr int kScanChunk = 2048;
+constexpr int kScanDirect = 64 * 1024;   // cells up to which a block adds up the counts before it
+__device__ __forceinline__ int block_sum256(int v) {
+    __shared__ int part[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w];
+    return t;
+}
+static __global__ void __launch_bounds__(256) k_cell_sums(const int* __restrict__ counts, int ncell, int* __restrict__ sums) {
+    pdl_enter();
+    const int b = blockIdx.x * kScanChunk;
+    int v = 0;
+#pragma unroll
+    for (int q = 0; q < kScanChunk / 256; ++q) {
+        const int i = b + q * 256 + threadIdx.x;
+        if (i < ncell) v += counts[i];
+    }
+    v = block_sum256(v);
+    if (threadIdx.x == 0) sums[blockIdx.x] = v;
+}
+static __global__ void __launch_bounds__(256) k_cell_scan(const int* __restrict__ counts, int ncell, int* __restrict__ start,
+                                                          const int* __restrict__ sums) {
+    pdl_enter();
+    const int b = blockIdx.x * kScanChunk, tid = threadIdx.x;
+    int before = 0;
+    if (sums) for (int i = tid; i < (int)blockIdx.x; i += 256) before += sums[i];
+    else {
+#pragma unroll 4
+        for (int i = tid; i < b / 4; i += 256) {
+            const int4 u = reinterpret_cast<const int4*>(counts)[i];
+            before += u.x + u.y + u.z + u.w;
+        }
+    }
+    constexpr int PER = kScanChunk / 256;   // 8: two 16-byte accesses per thread
+    const int i0 = b + tid * PER;
+    int v[PER], own = 0;
+    if (i0 + PER <= ncell) {
+        const int4 u = reinterpret_cast<const int4*>(counts + i0)[0], w = reinterpret_cast<const int4*>(counts + i0)[1];
+        v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) v[q] = i0 + q < ncell ? counts[i0 + q] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) own += v[q];
+    before = block_sum256(before);
+    // inclusive scan of the threads' sums
+    __shared__ int warp_tot[8];
+    int inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, inc, o);
+        if ((tid & 31) >= o) inc += u;
+    }
+    if ((tid & 31) == 31) warp_tot[tid >> 5] = inc;
+    __syncthreads();
+    int run = before + inc - own;
+    for (int w = 0; w < (tid >> 5); ++w) run += warp_tot[w];
+    if (i0 + PER < ncell) {
+        int o[PER];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) { o[q] = run; run += v[q]; }
+        reinterpret_cast<int4*>(start + i0)[0] = make_int4(o[0], o[1], o[2], o[3]);
+        reinterpret_cast<int4*>(start + i0)[1] = make_int4(o[4], o[5], o[6], o[7]);
+    } else {
+        for (int q = 0; q < PER && i0 + q < ncell; ++q) {
+            start[i0 + q] = run;
+            run += v[q];
+            if (i0 + q + 1 == ncell) start[ncell] = run;
+        }
+    }
+}
+
+// Also resets the cells' counts, consumed by the scan, for the corrector, which
+// counts the next step's cells (counts may be null).
 static __global__ void __launch_bounds__(256) k_cell_scatter(int n, const int* __restrict__ cell_id, const int* __restrict__ rank,
-                                                      const int* __restrict__ cell_start, int* __restrict__ perm) {
+                                                      const int* __restrict__ cell_start, int* __restrict__ perm,
+                                                      int* __restrict__ counts, int ncell) {
     pdl_enter();
     int a = gtid();
-    if (a >= n) return;
-    perm[cell_start[cell_id[a]] + rank[a]] = a;
+    if (a < n) perm[cell_start[cell_id[a]] + rank[a]] = a;
+    if (counts)
+        for (int c = a; c < ncell; c += gridDim.x * blockDim.x) counts[c] = 0;
 }
 
 // Insertion sort of each cell's (few) entries by original particle index, so
 // the visiting order, and with it every sum, depends neither on atomic timing
 // nor on the current state order (a download/upload restart is bit-identical).
-// The cell's count, consumed by the scan, is reset to zero for the corrector,
-// which counts the next step's cells.
+// A step without a reorder leaves this to the gather (sorted_slot).
 static __global__ void __launch_bounds__(256) k_cell_sort(int ncell, const int* __restrict__ cell_start,
-                                                   const int* __restrict__ orig, int* __restrict__ perm,
-                                                   int* __restrict__ counts) {
+                                                   const int* __restrict__ orig, int* __restrict__ perm) {
     pdl_enter();
     int c = gtid();
     if (c >= ncell) return;
-    counts[c] = 0;
     int b = cell_start[c], e = cell_start[c + 1];
     for (int i = b + 1; i < e; ++i) {
         int v = perm[i], ov = orig[v], j = i - 1;
         while (j >= b && orig[perm[j]] > ov) { perm[j + 1] = perm[j]; --j; }
         perm[j + 1] = v;
     }
+}
+
+// Sorted slot of the particle a, from the scattered cell list: its cell's first
+// slot plus the number of the cell's particles with a lower original index.
+__device__ __forceinline__ int sorted_slot(const int* __restrict__ scattered, const int* __restrict__ cell_id,
+                                           const int* __restrict__ cell_start, const int* __restrict__ orig, int a) {
+    const int c = cell_id[a], b = cell_start[c], e = cell_start[c + 1];
+    if (e - b == 1) return b;
+    const int o = orig[a];
+    int t = b;
+    for (int i = b; i < e; ++i) t += orig[scattered[i]] < o;
+    return t;
 }
 
 // ------------------------------------------------------------- integrators
@@ -263,24 +363,28 @@ __device__ __forceinline__ void count_fail(DevCounters* cnt, int slot, int fail)
 // leapfrog predictor (first_half, + DP on soil).  For soil also the in-step
 // Drucker-Prager return (declarations_sph.f90:1242-1247) on the state and the
 // stress/pressure record of the soil pass.  Bound by DRAM: it reads and writes
-// each field once, with every load before the first store.  Storing the half
+// each field once, with every load before the first store.  scattered: the
+// cell list before its cells are ordered; the gather then finds each
+// particle's slot itself and writes perm, which saves the sort's launch and pass
+// over the cells.  Storing the half
 // step as well (and reading it back in the corrector) took 53 us for the two
 // phases of 912,016 particles instead of 34, and the step 345 us instead of
 // 322; 5, 6 and 8 resident blocks spill and take 33, 36 and 38 us.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_gather(PhaseDev<T> P, SimConst c, int soil, int do_dp, int fh, int with_hs,
-                                                int fh_dp, DevCounters* cnt) {
+                                                int fh_dp, DevCounters* cnt, const int* __restrict__ scattered) {
     pdl_enter();
     int k = gtid();
     int fail0 = 0, fail = 0;
     if (k < P.n) {
-        const int a = P.perm[k];
+        const int a = scattered ? k : P.perm[k];   // by particle, which reads the state in order, or by slot
         const double2 x = P.x[a];
         double2 v = P.v[a];
         double rho = P.rho[a];
         const double mass = P.mass[a], h = with_hs ? P.hsml[a] : 0.0;
         const int sid = soil || fh ? P.sid[a] : 0, itype = soil || fh ? P.itype[a] : 0;
         const SceneTab& st = c.tab[sid];
+        if (scattered) k = sorted_slot(scattered, P.cell_id, P.cell_start, P.orig, a);
         double p = 0.0, sxx = 0.0, sxy = 0.0, syy = 0.0, cc = 0.0, vof = 0.0;
         if (soil) { p = P.p[a]; sxx = P.sxx[a]; sxy = P.sxy[a]; syy = P.syy[a]; cc = P.c[a]; vof = P.vof[a]; }
         if (fh) {
@@ -301,6 +405,7 @@ __global__ void __launch_bounds__(256, 4) k_gather(PhaseDev<T> P, SimConst c, in
             rb.itype = (T)itype; rb.aux = T(0);
             P.recB[k] = rb;
         }
+        if (scattered) P.perm[k] = a;
         P.xs[k] = x;
         if (with_hs) P.hs[k] = h;
         RecA<T> ra;
@@ -1100,39 +1205,11 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
 // The step's counters and the batch's sticky flags as the host reads them.
 struct CounterMirror { DevCounters c; int sticky[4]; };
 
-// Sticky per-batch flags: a pair list above max_interaction (the reference
-// stops there, m_particles.f90:992-993) and non-finite positions.  With a
-// mirror (mapped pinned host memory) the step's counters and the flags are
-// also written there, so the host reads them after its synchronisation with
-// no copy of its own.
-static __global__ void k_check(const DevCounters* __restrict__ c, int* __restrict__ sticky, unsigned long long cap,
-                               CounterMirror* __restrict__ mirror) {
-    pdl_enter();
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const int f[3] = {c->pairs[0] / 2 > cap || c->pairs[1] / 2 > cap || c->pairs[2] > cap, c->nonfinite != 0,
-                          c->timeout != 0};
-        for (int i = 0; i < 3; ++i)
-            if (f[i]) sticky[i] = 1;
-        if (mirror) {
-            mirror->c = *c;
-            for (int i = 0; i < 3; ++i)
-                if (f[i]) mirror->sticky[i] = 1;
-            __threadfence_system();
-        }
-    }
-}
-
-// ------------------------------------------------------- layout transforms
-// Every persistent field of a phase permuted into the current cell order in
-// one launch: dst_i[k] = src_i[perm[k]].
-struct PermField { const void* src; void* dst; int bytes; int pad; };
-struct PermList { int count; int pad; PermField f[44]; };
-// Per-step counters to their initial values (a kernel, so that it can live in a graph).
-// take_next: the step's cell keys were counted by the previous step's
-// corrector, with its clamped and non-finite positions.
-static __global__ void k_reset_counters(DevCounters* c, int take_next) {
-    pdl_enter();
-    int i = threadIdx.x;
+// The counters' values at the start of a step.  take_next: the step's cell keys
+// were counted by the corrector of the step before, with its clamped and
+// non-finite positions.
+__device__ __forceinline__ void reset_counters(DevCounters* c, int take_next) {
+    const int i = threadIdx.x;
     if (i < 3) c->pairs[i] = 0ull;
     if (i < 2) { c->maxiac[i] = 0; c->miniac[i] = 0x7fffffff; c->noiac[i] = 0; }
     if (i < 4) c->nfail[i] = 0;
@@ -1143,7 +1220,45 @@ static __global__ void k_reset_counters(DevCounters* c, int take_next) {
         c->overflow = 0; c->timeout = 0;
     }
 }
+static __global__ void k_reset_counters(DevCounters* c, int take_next) {
+    pdl_enter();
+    reset_counters(c, take_next);
+}
 
+// Sticky per-batch flags: a pair list above max_interaction (the reference
+// stops there, m_particles.f90:992-993) and non-finite positions.  With a
+// mirror (mapped pinned host memory) the step's counters and the flags are
+// also written there, so the host reads them after its synchronisation with
+// no copy of its own, and (next != 0) the counters are reset for the next step,
+// whose cells the corrector has counted.  One warp, a word per lane.
+static __global__ void k_check(DevCounters* __restrict__ c, int* __restrict__ sticky, unsigned long long cap,
+                               CounterMirror* __restrict__ mirror, int next) {
+    pdl_enter();
+    const int i = threadIdx.x;
+    constexpr int W = (int)(sizeof(DevCounters) / sizeof(int));
+    static_assert(sizeof(DevCounters) % sizeof(int) == 0 && W <= 32, "a counter word per lane");
+    int word = 0;
+    if (mirror && i < W) word = reinterpret_cast<const int*>(c)[i];
+    bool flag = false;
+    if (i == 0) flag = c->pairs[0] / 2 > cap || c->pairs[1] / 2 > cap || c->pairs[2] > cap;
+    if (i == 1) flag = c->nonfinite != 0;
+    if (i == 2) flag = c->timeout != 0;
+    if (flag) {
+        sticky[i] = 1;
+        if (mirror) mirror->sticky[i] = 1;
+    }
+    if (mirror) {
+        if (i < W) reinterpret_cast<int*>(&mirror->c)[i] = word;
+        __syncwarp();
+        if (next) reset_counters(c, 1);
+    }
+}
+
+// ------------------------------------------------------- layout transforms
+// Every persistent field of a phase permuted into the current cell order in
+// one launch: dst_i[k] = src_i[perm[k]].
+struct PermField { const void* src; void* dst; int bytes; int pad; };
+struct PermList { int count; int pad; PermField f[44]; };
 static __global__ void __launch_bounds__(256) k_permute_all(int n, const int* __restrict__ perm, PermList L) {
     pdl_enter();
     int k = gtid();
