@@ -130,13 +130,15 @@ static __global__ void __launch_bounds__(256) k_cell_count(const double2* __rest
 // Exclusive scan of the cells' counts, start[ncell] = the total: each block
 // scans a chunk of kScanChunk counts on top of the sum of all counts before it,
 // taken from the chunk sums of k_cell_sums or, for few cells, from the counts
-// themselves (one launch instead of two below 64k cells).  Bound: launches and
+// themselves (one launch instead of two).  us per step with and without the chunk
+// sums: 3.5k cells 30.6, 30.2; 15k 22.1, 22.4; 28k 24.0, 25.2; 52k 26.3, 29.4;
+// 100k 28.3, 34.3: the line is 16k.  Bound: launches and
 // their latency.  With the cells ordered inside the gather and the counters
 // reset by the step's check, us per step before and after: 7.4k particles 33.4,
 // 28.4; 150k 95, 91; 190k 77, 70; 330k 172, 165; 912k 325, 316; the ensemble's
 // dry group 121, 104.
 constexpr int kScanChunk = 2048;
-constexpr int kScanDirect = 64 * 1024;   // cells up to which a block adds up the counts before it
+constexpr int kScanDirect = 16 * 1024;   // cells up to which a block adds up the counts before it
 __device__ __forceinline__ int block_sum256(int v) {
     __shared__ int part[8];
 #pragma unroll

@@ -26,7 +26,7 @@ def column(precision, span):
     return s
 
 
-# about 0.9k, 2k, 30k, 64k and 90k cells at 8 per support radius; 1k at whole cells
+# from a few thousand cells to several times 10,000 at 8 per support radius; few at whole cells
 @pytest.mark.parametrize("span,split", [(0.5, 8), (1, 8), (8, 8), (21, 8), (30, 8), (4, 1)])
 @pytest.mark.parametrize("precision", [SPHG_FP64, SPHG_FP32])
 def test_sort_and_gather_give_the_same_order(cuda_ok, precision, span, split):
