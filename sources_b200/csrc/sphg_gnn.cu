@@ -483,27 +483,39 @@ __global__ void k_node_concat_bwd(const float* __restrict__ d, float* __restrict
 // Huber loss (squared error up to |d| = delta, linear beyond; plain squared
 // error for delta <= 0) over the rows with mask != 0, first nout columns of
 // pred (row stride ld), scaled by inv_count; dpred = d loss / d pred (zero
-// elsewhere)
-__global__ void k_mse(const float* __restrict__ pred, int ld, const float* __restrict__ target, int nout,
-                      const float* __restrict__ mask, long long rows, float inv_count, float delta,
-                      float* __restrict__ dpred, float* __restrict__ loss) {
+// elsewhere).  Bound by the writes of dpred: a block adds its terms up and
+// issues one atomic (23k rows of 128: 22 us; with one per term 69).
+__global__ void __launch_bounds__(256) k_mse(const float* __restrict__ pred, int ld, const float* __restrict__ target, int nout,
+                                             const float* __restrict__ mask, long long rows, float inv_count, float delta,
+                                             float* __restrict__ dpred, float* __restrict__ loss) {
+    __shared__ float part[8];
     const long long i = gid();
-    if (i >= rows * ld) return;
-    const long long r = i / ld;
-    const int c = (int)(i % ld);
-    float g = 0.f;
-    if (c < nout && mask[r] != 0.f) {
-        const float d = pred[i] - target[r * nout + c];
-        const float a = fabsf(d);
-        if (delta <= 0.f || a <= delta) {
-            g = 2.f * d * inv_count;
-            atomicAdd(loss, d * d * inv_count);
-        } else {
-            g = copysignf(2.f * delta, d) * inv_count;
-            atomicAdd(loss, delta * (2.f * a - delta) * inv_count);
+    float t = 0.f;
+    if (i < rows * ld) {
+        const long long r = i / ld;
+        const int c = (int)(i - r * ld);
+        float g = 0.f;
+        if (c < nout && mask[r] != 0.f) {
+            const float d = pred[i] - target[r * nout + c];
+            const float a = fabsf(d);
+            if (delta <= 0.f || a <= delta) {
+                g = 2.f * d * inv_count;
+                t = d * d * inv_count;
+            } else {
+                g = copysignf(2.f * delta, d) * inv_count;
+                t = delta * (2.f * a - delta) * inv_count;
+            }
         }
+        dpred[i] = g;
     }
-    dpred[i] = g;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) t += part[w];
+        if (t != 0.f) atomicAdd(loss, t);
+    }
 }
 
 // Adam (Kingma & Ba 2015) on fp32 master weights [rows x cols]; rows at or
