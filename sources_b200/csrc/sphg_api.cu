@@ -566,7 +566,8 @@ struct Engine : EngineBase {
         rc |= alloc(&D.countiac, N); rc |= alloc(&D.cell_id, N); rc |= alloc(&D.cell_fill, N); rc |= alloc(&D.perm, N);
         rc |= alloc(&scattered[ph], N);
         rc |= alloc(&D.xs, N); rc |= alloc(&D.hs, N);
-        rc |= alloc(&D.recA, N); rc |= alloc(&D.recA2, N); rc |= alloc(&D.recB, N); rc |= alloc(&D.hmask, N);
+        rc |= alloc(&D.recA, N); rc |= alloc(&D.recA2, N); rc |= alloc(&D.recB, N);
+        rc |= alloc(&D.hmask, N + (N & 1));   // whole lane pairs (k_water_pass_a2)
         if (rc) return SPHG_ERR_CUDA;
         for (auto& f : field_refs(ph)) {
             char* q = nullptr;

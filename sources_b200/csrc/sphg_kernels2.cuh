@@ -158,11 +158,11 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_A2) k_water_pass_a2(Phase
     });
     const int hits = p.mine(hits0, hits1);
     const float con_ = p.mine(con), dl_ = p.mine(dl), ta_ = p.mine(ta), tb_ = p.mine(tb), tc_ = p.mine(tc);
+    if (p.v0) P.hmask[p.k] = mask;   // a lane without a particle of its own still has its half of the pair's candidates
     if (p.valid) {
         // delta_sph: 2 delta h c (rho_a - rho_b), c of the previous EOS call
         const float d = c.artificial_density ? -2.0f * K.ks * (float)(c.delta * (double)K.h * P.c[P.perm[p.k]]) * dl_ : 0.0f;
         const float c23 = K.ks * (2.0f / 3.0f);
-        P.hmask[p.k] = mask;
         water_a_finish<float, false>(P, c, p.k, -K.ks * con_, d, c23 * (2.0f * ta_ - tb_), K.ks * tc_, c23 * (2.0f * tb_ - ta_),
                                      0.0f, hits);
     }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_B2) k_water_pass_b2(Phase
             dvf = fma2(mul2(vb, add2(fb, nphi)), s, dvf);
             if (qb.itype < 0.0f) wall_pair(K, rr, dx, dy, h0 && real0, h1 && real1, ex, ey);
         };
-        const uint4 mask = p.valid ? P.hmask[p.k] : make_uint4(0u, 0u, 0u, 0u);   // recorded by the step's first water pass
+        const uint4 mask = p.v0 ? P.hmask[p.k] : make_uint4(0u, 0u, 0u, 0u);   // recorded by the step's first water pass
         visit_pairs<true>(P, g, p, &cnt->timeout, [&](const Runs3& r, const double2* xs, const RecA<float>* RA,
                                                            const RecB<float>* RB, int s0, int s1, bool a0, bool a1) {
             pair_replay(r, p.lane, K.thr, xs, p.x0, p.x1, s0, s1, a0, a1, mask,
