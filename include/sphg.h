@@ -172,7 +172,8 @@ int sphg_create(const sphg_params* p, int n_phase, sphg_ctx** out);
  * and kept until sphg_destroy; pinned host arrays move at the link's speed,
  * pageable ones through page-locked buffers that the contexts share (at most
  * 8 MB, freed with the last context), with up to three helper threads that
- * end before the call returns. */
+ * end before the call returns (none on cudaStreamPerThread, which is another
+ * stream in each thread). */
 int sphg_upload_phase(sphg_ctx* ctx, int phase, const sphg_phase_host* v);
 
 /* Right-hand side only: single_step (declarations_sph.f90:1131), or
