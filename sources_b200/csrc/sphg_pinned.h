@@ -6,7 +6,6 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -176,7 +175,7 @@ struct PinnedCopies {
         for (int w = 1; w < nw; ++w) {
             try {
                 th[w] = std::thread([&, w] { if (work(slot[w], w, nw, s, dev, total, piece, up, st)) bad = 1; });
-            } catch (const std::system_error&) {
+            } catch (...) {
                 here |= 1 << w;
             }
         }
@@ -184,6 +183,7 @@ struct PinnedCopies {
             if ((here >> w & 1) && work(slot[w], w, nw, s, dev, total, piece, up, st)) bad = 1;
         for (int w = 1; w < nw; ++w)
             if (th[w].joinable()) th[w].join();
+        if (bad) cudaStreamSynchronize(st);   // a copy may be in flight whose event was not recorded
         for (int w = 0; w < nw; ++w) release(slot[w]);
         return bad;
     }

@@ -150,3 +150,18 @@ def test_copies_follow_the_callers_stream(fake, stream, up, total):
     alone = total < (4 << 20) or mine
     fake(f"size_t threads = 0; if (transfer({stream}, {total}, {up}, &threads)) return 1;"
          f"if (threads != {1 if alone else 4}) return bad(\"threads\");")
+
+
+@pytest.mark.parametrize("up", [0, 1])
+@pytest.mark.parametrize("record", [0, 1, 5, 17])
+def test_a_failed_transfer_leaves_nothing_in_flight(fake, up, record):
+    """The buffers go back to the pool when the call returns: no copy may still use one, whichever call failed."""
+    fake(f"""const size_t total = 70 << 20;
+    PinnedCopies pc;
+    std::vector<std::vector<char>> h(1, std::vector<char>(total));
+    std::vector<char> dev(total);
+    fail_record = {record};
+    if (pc.run(segs(h), dev.data(), total, {up}, (cudaStream_t)64, 0) != 1) return bad("status");
+    for (auto& k : in_flight) if (k.second) return bad("a copy is in flight");
+    size_t threads;
+    if (transfer((cudaStream_t)65, total, {up}, &threads)) return 1;""")
