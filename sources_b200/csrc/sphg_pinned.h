@@ -33,6 +33,7 @@ struct PinnedCopies {
     // One worker's two buffers, lent to one transfer at a time.  The slots are
     // shared by the contexts of the process (making one takes as long as ten
     // small transfers), at most kSlots of them, and freed with the last context.
+    // At the limit an idle slot of another device gives way to a new one.
     struct Slot {
         int device = 0;
         char* buf[2] = {nullptr, nullptr};
@@ -50,13 +51,17 @@ struct PinnedCopies {
     }
     static void destroy(Slot* s) {
         for (int b = 0; b < 2; ++b) {
+            if (s->ev[b]) {
+                cudaEventSynchronize(s->ev[b]);   // the last pieces of an upload may still be queued
+                cudaEventDestroy(s->ev[b]);
+            }
             if (s->buf[b]) cudaFreeHost(s->buf[b]);
-            if (s->ev[b]) cudaEventDestroy(s->ev[b]);
         }
         delete s;
     }
     static Slot* acquire(int device) {
         Pool& P = pool();
+        Slot* other = nullptr;
         {
             std::lock_guard<std::mutex> l(P.m);
             for (size_t i = 0; i < P.idle.size(); ++i)
@@ -65,9 +70,15 @@ struct PinnedCopies {
                     P.idle.erase(P.idle.begin() + (long)i);
                     return s;
                 }
-            if (P.made >= kSlots) return nullptr;
-            ++P.made;
+            if (P.made < kSlots) {
+                ++P.made;
+            } else {
+                if (P.idle.empty()) return nullptr;
+                other = P.idle.back();
+                P.idle.pop_back();
+            }
         }
+        if (other) destroy(other);
         Slot* s = new Slot();
         s->device = device;
         bool ok = true;

@@ -165,3 +165,34 @@ def test_a_failed_transfer_leaves_nothing_in_flight(fake, up, record):
     for (auto& k : in_flight) if (k.second) return bad("a copy is in flight");
     size_t threads;
     if (transfer((cudaStream_t)65, total, {up}, &threads)) return 1;""")
+
+
+def test_idle_buffers_serve_every_device(fake):
+    """Eight pairs of buffers in all: those that one device's transfers made and left idle serve another's."""
+    fake("""const size_t total = 6 << 20;
+    PinnedCopies pc;
+    for (int dev = 0; dev < 3; ++dev) {
+        std::vector<PinnedCopies::Slot*> s;
+        for (int i = 0; i < PinnedCopies::kSlots; ++i) {
+            s.push_back(PinnedCopies::acquire(dev));
+            if (!s.back() || s.back()->device != dev) return bad("no buffers");
+        }
+        if (PinnedCopies::acquire(dev) || PinnedCopies::acquire(dev + 1)) return bad("more buffers than the limit");
+        if (pinned_mem.size() != 2 * PinnedCopies::kSlots) return bad("page-locked memory");
+        for (auto* p : s) PinnedCopies::release(p);
+    }
+    std::vector<std::vector<char>> h(1, std::vector<char>(total));
+    std::vector<char> dev(total);
+    if (pc.run(segs(h), dev.data(), total, false, (cudaStream_t)64, 5) != 0) return bad("run");
+    if (freed_busy) return bad("a buffer was freed with a copy in flight");""")
+
+
+def test_idle_buffers_are_freed_after_their_copies(fake):
+    """An upload returns with its last pieces queued; another device's transfer frees those buffers only then."""
+    fake("""const size_t total = 70 << 20;
+    PinnedCopies pc;
+    std::vector<std::vector<char>> h(1, std::vector<char>(total));
+    std::vector<char> dev(total);
+    if (pc.run(segs(h), dev.data(), total, true, (cudaStream_t)64, 0) != 0) return bad("run");
+    for (int i = 0; i < PinnedCopies::kSlots; ++i) if (!PinnedCopies::acquire(1)) return bad("no buffers");
+    if (freed_busy) return bad("a buffer was freed with a copy in flight");""")
