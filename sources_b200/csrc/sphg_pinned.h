@@ -114,10 +114,10 @@ struct PinnedCopies {
     }
     PinnedCopies(const PinnedCopies&) = delete;
     PinnedCopies& operator=(const PinnedCopies&) = delete;
-    static bool pageable(const void* p) {
+    static cudaMemoryType type(const void* p) {
         cudaPointerAttributes a;
-        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return true; }
-        return a.type == cudaMemoryTypeUnregistered;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return cudaMemoryTypeUnregistered; }
+        return a.type;
     }
     // host side of bytes [o, o + n) of the device range
     static void host_part(const std::vector<Seg>& s, size_t o, size_t n, char* pin, bool up) {
@@ -166,10 +166,17 @@ struct PinnedCopies {
         host_part(s, o, n, slot->buf[b], false);
         return 0;
     }
-    // 0 done (upwards: the host arrays are no longer read), 1 error, -1 not taken (page-locked arrays, or no buffer)
+    // 0 done (upwards: the host arrays are no longer read), 1 error, -1 not taken (page-locked arrays only, a
+    // device address among them, or no buffer)
     int run(const std::vector<Seg>& s, char* dev, size_t total, bool up, cudaStream_t st, int device) {
         bool any = false;
-        for (const Seg& g : s) any = any || (g.h0 && pageable(g.h0)) || (g.h1 && pageable(g.h1));
+        for (const Seg& g : s) {
+            for (const char* h : {g.h0, g.h1}) {
+                const cudaMemoryType t = h ? type(h) : cudaMemoryTypeHost;
+                if (t == cudaMemoryTypeDevice) return -1;
+                any = any || t == cudaMemoryTypeUnregistered;
+            }
+        }
         // cudaStreamPerThread is another stream in each thread: the calling thread then works alone, and uploads,
         // which one thread moves no faster than the driver, stay with the driver
         const bool shared = st != cudaStreamPerThread;

@@ -196,3 +196,15 @@ def test_idle_buffers_are_freed_after_their_copies(fake):
     if (pc.run(segs(h), dev.data(), total, true, (cudaStream_t)64, 0) != 0) return bad("run");
     for (int i = 0; i < PinnedCopies::kSlots; ++i) if (!PinnedCopies::acquire(1)) return bad("no buffers");
     if (freed_busy) return bad("a buffer was freed with a copy in flight");""")
+
+
+@pytest.mark.parametrize("up,total", [(0, 1 << 20), (1, 70 << 20)])
+def test_device_arrays_stay_with_the_driver(fake, up, total):
+    """A device address among the arrays is for the driver to move or refuse; the host never touches it."""
+    fake(f"""PinnedCopies pc;
+    std::vector<std::vector<char>> h(3, std::vector<char>({total}));
+    std::vector<char> dev(3 * {total});
+    auto s = segs(h);
+    s[1].h0 = (char*)4096;
+    device_ptrs.insert(s[1].h0);
+    if (pc.run(s, dev.data(), dev.size(), {up}, (cudaStream_t)64, 0) != -1) return bad("taken");""")
