@@ -849,8 +849,13 @@ struct Engine : EngineBase {
         const int* sums = ncell > kScanDirect ? chunk_sums[ph] : nullptr;
         if (sums && (rc = launch_pdl("cell_sums", k_cell_sums, chunks, 256, 0, (const int*)counts[ph], ncell, chunk_sums[ph])))
             return rc;
-        if ((rc = launch_pdl("cell_scan", k_cell_scan, chunks, 256, 0, (const int*)counts[ph], ncell, D.cell_start, sums))) return rc;
-        if ((rc = launch_pdl("cell_scatter", k_cell_scatter, blocks(D.n, 256), 256, 0, D.n, (const int*)D.cell_id,
+        const int scanned = sums && chunks > kSumsDirect;
+        if (scanned && (rc = launch_pdl("sums_scan", k_sums_scan, 1, 1024, 0, chunk_sums[ph], chunks))) return rc;
+        if ((rc = launch_pdl("cell_scan", k_cell_scan, chunks, 256, 0, (const int*)counts[ph], ncell, D.cell_start, sums, scanned)))
+            return rc;
+        // a thread per particle, and no more than 16 cells a thread to clear, up to a full GPU
+        const int nb = std::max(blocks(D.n, 256), std::min(blocks(ncell, 16 * 256), 8 * 148));
+        if ((rc = launch_pdl("cell_scatter", k_cell_scatter, nb, 256, 0, D.n, (const int*)D.cell_id,
                              (const int*)D.cell_fill, (const int*)D.cell_start, sorted ? D.perm : scattered[ph], counts[ph], ncell)))
             return rc;
         if (!sorted) return 0;

@@ -137,8 +137,14 @@ static __global__ void __launch_bounds__(256) k_cell_count(const double2* __rest
 // reset by the step's check, us per step before and after: 7.4k particles 33.4,
 // 28.4; 150k 95, 91; 190k 77, 70; 330k 172, 165; 912k 325, 316; the ensemble's
 // dry group 121, 104.
+// Above kSumsDirect chunks the blocks' reads of all sums before theirs, which grow
+// with the square of the cells, cost more than a launch that scans the sums:
+// us per step of 6.6k particles without and with it, 4M cells 34.0, 34.5; 8M 45.5,
+// 45.5; 16M 71.0, 69.7; 69M 284, 238; 180M 1,020, 573.  Bound there: HBM, four
+// passes over the cells (counts read twice and cleared, starts written).
 constexpr int kScanChunk = 2048;
 constexpr int kScanDirect = 16 * 1024;   // cells up to which a block adds up the counts before it
+constexpr int kSumsDirect = 4096;        // chunks up to which a block adds up the chunk sums before it; above, one block scans them first
 __device__ __forceinline__ int block_sum256(int v) {
     __shared__ int part[8];
 #pragma unroll
@@ -163,12 +169,49 @@ static __global__ void __launch_bounds__(256) k_cell_sums(const int* __restrict_
     v = block_sum256(v);
     if (threadIdx.x == 0) sums[blockIdx.x] = v;
 }
+// The chunk sums replaced by the sum of all sums before each, by one block, 4,096 at a time.
+static __global__ void __launch_bounds__(1024) k_sums_scan(int* __restrict__ sums, int n) {
+    pdl_enter();
+    __shared__ int warp_tot[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int carry = 0;
+    for (int b = 0; b < n; b += 4096) {
+        const int i0 = b + tid * 4;
+        int v[4], own = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { v[q] = i0 + q < n ? sums[i0 + q] : 0; own += v[q]; }
+        int inc = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (lane == 31) warp_tot[warp] = inc;
+        __syncthreads();
+        int w = warp_tot[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        int run = carry + inc - own + (warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0);
+        carry += __shfl_sync(0xffffffffu, w, 31);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (i0 + q < n) sums[i0 + q] = run;
+            run += v[q];
+        }
+        __syncthreads();   // warp_tot is read before the next tile's sums replace it
+    }
+}
+// sums: null, or the chunk sums (scanned: already scanned by k_sums_scan)
 static __global__ void __launch_bounds__(256) k_cell_scan(const int* __restrict__ counts, int ncell, int* __restrict__ start,
-                                                          const int* __restrict__ sums) {
+                                                          const int* __restrict__ sums, int scanned) {
     pdl_enter();
     const int b = blockIdx.x * kScanChunk, tid = threadIdx.x;
     int before = 0;
-    if (sums) for (int i = tid; i < (int)blockIdx.x; i += 256) before += sums[i];
+    if (sums && scanned) before = tid == 0 ? sums[blockIdx.x] : 0;
+    else if (sums) for (int i = tid; i < (int)blockIdx.x; i += 256) before += sums[i];
     else {
 #pragma unroll 4
         for (int i = tid; i < b / 4; i += 256) {
@@ -217,7 +260,12 @@ static __global__ void __launch_bounds__(256) k_cell_scan(const int* __restrict_
 }
 
 // Also resets the cells' counts, consumed by the scan, for the corrector, which
-// counts the next step's cells (counts may be null).
+// counts the next step's cells (counts may be null).  The grid has a thread per
+// particle and, for grids of many more cells, one per 16 cells: cleared by the
+// particles' blocks alone, a step of 6.6k particles took 28.8 us at 1M cells and
+// 143 at 16M; with these, 26.4 and 69.7.  (One thread per 4 cells changes the
+// small steps' block counts, and with them where the next passes' blocks land:
+// 32.4 us for the FP32 step of 6.6k particles instead of 28.8.)
 static __global__ void __launch_bounds__(256) k_cell_scatter(int n, const int* __restrict__ cell_id, const int* __restrict__ rank,
                                                       const int* __restrict__ cell_start, int* __restrict__ perm,
                                                       int* __restrict__ counts, int ncell) {
