@@ -524,7 +524,7 @@ __device__ __forceinline__ void water_sum_finish(const PhaseDev<T>& P, const Sim
     const int a = P.perm[k];
     const T rho = num / wi;
     const double mass = P.mass[a];
-    if (c.half) P.rho_min[a] = P.rho[a];   // the corrector integrates from it
+    if (c.half && !c.summation_density) P.rho_min[a] = P.rho[a];   // the corrector integrates from it
     P.rho[a] = (double)rho;
     P.drho[a] = -rho * (sx / rho + sy / rho);
     RecA<T> r2;
