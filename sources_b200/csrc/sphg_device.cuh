@@ -270,12 +270,24 @@ __device__ __forceinline__ int warp_min(int v) {
 // loop (every pair of a particle shares one h when all h are equal).
 // eval() returns W and the radial factor s with grad W = s * dx, so that
 // dx . grad W = s * r^2.  r and 1/r come from one rsqrt and q from a product
-// with 1/h (in FP64 too: a sqrt and two divisions per pair, each a serial chain
-// of FP64 operations, were a fifth of the FP64 passes).
+// with 1/h; in FP64 each is then corrected by its residual (quot_, rcp_near),
+// which gives the square root and quotients of the reference's expression to the
+// last bit but for rare ties: a sqrt and two divisions per pair, each a serial
+// chain of FP64 operations, were a fifth of the FP64 passes.
 template <typename T> __device__ __forceinline__ T rcp_(T x) { return T(1) / x; }
 template <> __device__ __forceinline__ float rcp_<float>(float x) { return __frcp_rn(x); }
 template <typename T> __device__ __forceinline__ T div_(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ float div_<float>(float a, float b) { return __fdividef(a, b); }
+
+// 1 / b and a / b in FP64 from x close to 1 / b: one Newton step for the
+// reciprocal, and the product corrected by its exact residual for the quotient
+// (P. Markstein, IBM J. Res. Dev. 34, 1990).  Each is the correctly rounded value
+// in all but rare cases, and at most one ulp off in those.
+__device__ __forceinline__ double rcp_near(double b, double x) { return fma(fma(-b, x, 1.0), x, x); }
+__device__ __forceinline__ double quot_(double a, double b, double x) {
+    const double q = a * x;
+    return fma(fma(-q, b, a), x, q);
+}
 
 // x^p of the wall force: pow in FP64; in FP32 the fast exp2(p log2 x) (a few
 // ulp at the exponents and ranges of the wall force, p = 12 and 4, x >= 1)
@@ -303,14 +315,18 @@ struct KernelConst {
     // r2 = dx^2 + dy^2 of the pair
     __device__ __forceinline__ void eval(T r2, T& w, T& s) const {
         T r, rinv;
-        if (sizeof(T) == 8) {
-            rinv = (T)rsqrt(fmax((double)r2, 1e-300));
+        T q;
+        if constexpr (sizeof(T) == 8) {
+            rinv = rsqrt(fmax(r2, 1e-300));
             r = r2 * rinv;
+            r = fma(fma(-r, r, r2), 0.5 * rinv, r);
+            rinv = rcp_near(r, rinv);
+            q = quot_(r, h, inv_h);
         } else {
             rinv = (T)rsqrtf((float)fmaxf((float)r2, 1e-30f));
             r = r2 * rinv;
+            q = r * inv_h;
         }
-        const T q = r * inv_h;
         w = T(0); s = T(0);
         if (SKF == 1) {
             if (q <= T(1)) {

@@ -926,12 +926,13 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
         d3 = fma2(splat2(vb), mul2(s_b, splat2(gr.y)), d3);
         const T2 dv = sub2(va, vb2);                              // v_a - v_b
         const T mb = vb * rb.rho;
-        // 1 / mean density (art_visc and av_vel); in FP64 from one reciprocal with 1 / (r^2 + etq^2 h^2)
-        T irho, iden = T(0);
+        // 1 / mean density (art_visc and av_vel); in FP64 from one division with 1 / (r^2 + etq^2 h^2), then corrected
+        T irho, iden = T(0), den = T(0);
         if constexpr (sizeof(T) == 8) {
-            const T mr = T(0.5) * (ra.rho + rb.rho), den = fmax(rr + mh * mh * etq2, T(1e-300));
+            const T mr = T(0.5) * (ra.rho + rb.rho);
+            den = fmax(rr + mh * mh * etq2, T(1e-300));
             const T inv = T(1) / (mr * den);
-            irho = inv * den;
+            irho = rcp_near(mr, inv * den);
             iden = inv * mr;
         } else {
             irho = rcp_<T>(T(0.5) * (ra.rho + rb.rho));
@@ -939,7 +940,9 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
         if (visc) {
             const T vr = dv.x * dx + dv.y * dy;
             if (vr < T(0)) {
-                const T muv = sizeof(T) == 8 ? mh * vr * iden : div_<T>(mh * vr, rr + mh * mh * etq2);
+                T muv;
+                if constexpr (sizeof(T) == 8) muv = quot_(mh * vr, den, iden);
+                else muv = div_<T>(mh * vr, rr + mh * mh * etq2);
                 const T mc = T(0.5) * (qa.c + qb.c);
                 const T piv = ((beta * muv - alpha * mc) * muv) * irho;
                 av = fma2(splat2(-mb), mul2(splat2(piv), gr), av);
@@ -1146,15 +1149,21 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
         const T du = rb.vx - ra.vx, dv = rb.vy - ra.vy;   // v_b - v_a
         const T vb = rb.vol, mb = vb * rb.rho;
         const T e = T(2) * sr;                            // 2 (dx . grad W) / r^2
-        // in FP64, 1 / mean density, 1 / (r^2 + etq^2 h^2) and 1 / rho_b from one reciprocal
-        T irho64 = T(0), iden64 = T(0), irb64 = T(0);
+        // in FP64, 1 / mean density, 1 / (r^2 + etq^2 h^2) and 1 / rho_b from one division (corrected where they are used)
+        T irho64 = T(0), iden64 = T(0), irb64 = T(0), den = T(0);
+        const T mr = T(0.5) * (ra.rho + rb.rho);
         if constexpr (sizeof(T) == 8) {
-            const T mr = T(0.5) * (ra.rho + rb.rho), den = fmax(rr + mh * mh * etq2, T(1e-300));
+            den = fmax(rr + mh * mh * etq2, T(1e-300));
             const T md = mr * den, inv = T(1) / (md * rb.rho);
             irb64 = inv * md;
             irho64 = inv * (den * rb.rho);
             iden64 = inv * (mr * rb.rho);
         }
+        // a / mean density
+        auto over_mr = [&](T a) {
+            if constexpr (sizeof(T) == 8) return quot_(a, mr, irho64);
+            else return div_<T>(a, mr);
+        };
         con -= mb * (du * gx + dv * gy);
         if (dens) dl += pref_old * vb * ((ra.rho - rb.rho) * e);
         txx += vb * (c23 * (T(2) * du * gx - dv * gy));
@@ -1170,7 +1179,9 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
             s2y += vb * ((faxy + qb.sxy) * gx);
             s3y += vb * ((fayy + qb.syy) * gy);
         } else {            // df3: m_b (f_a/rho_a^2 + f_b/rho_b^2) gradW
-            const T irb = sizeof(T) == 8 ? irb64 : rcp_<T>(rb.rho);
+            T irb;
+            if constexpr (sizeof(T) == 8) irb = rcp_near(rb.rho, irb64);
+            else irb = rcp_<T>(rb.rho);
             const T ib = qb.vof * irb * irb;
             const T pp = fap * ira2 + qb.p * ib;
             s1x += mb * (pp * gx); s1y += mb * (pp * gy);
@@ -1185,10 +1196,10 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
         if (visc) {
             const T vr = -(du * dx + dv * dy);
             if (vr < T(0)) {
-                const T muv = sizeof(T) == 8 ? mh * vr * iden64 : div_<T>(mh * vr, rr + mh * mh * etq2);
-                const T mrho = T(0.5) * (ra.rho + rb.rho);
-                const T pv = (beta * muv - alpha * cs) * muv;
-                const T piv = sizeof(T) == 8 ? pv * irho64 : div_<T>(pv, mrho);
+                T muv;
+                if constexpr (sizeof(T) == 8) muv = quot_(mh * vr, den, iden64);
+                else muv = div_<T>(mh * vr, rr + mh * mh * etq2);
+                const T piv = over_mr((beta * muv - alpha * cs) * muv);
                 avx -= mb * (piv * gx);
                 avy -= mb * (piv * gy);
             }
@@ -1209,7 +1220,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
             }
         }
         if (xsph) {
-            const T q = sizeof(T) == 8 ? mb * w * irho64 : div_<T>(mb * w, (ra.rho + rb.rho) / T(2));
+            const T q = over_mr(mb * w);
             xsx += q * du;
             xsy += q * dv;
         }
