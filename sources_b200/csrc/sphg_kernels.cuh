@@ -579,24 +579,27 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
     count_stats(cnt, 0, 0, hits, finish);
 }
 
-// r^3 to within rounding: the product and the rounding errors of its factors.
+// The powers of the Tait equation, r^gamma - 1, and of the sound speed, r^3.  FP64
+// calls pow, as the reference does.  The single-precision mode (whose equation
+// of state is in FP64 all the same) takes gamma = 7, the exponent of water, and the cube
+// as products with their rounding errors carried along: no further from the
+// exact value than pow, which took 250 instructions a call (an eighth of its
+// water_pass_a's).  Infinite products stand alone (their errors are NaN).
+template <typename T>
 __device__ __forceinline__ double cube(double r) {
-    const double r2 = r * r, e2 = fma(r, r, -r2), r3 = r2 * r;
-    return r3 + (fma(r2, r, -r3) + e2 * r);
+    if (sizeof(T) == 8) return pow(r, 3.0);
+    const double r2 = r * r, r3 = r2 * r;
+    if (isinf(r3)) return r3;
+    return r3 + (fma(r2, r, -r3) + fma(r, r, -r2) * r);
 }
-// r^gamma - 1 of the Tait equation.  gamma = 7, the exponent of water, as
-// products with their rounding errors carried along: closer to the exact value
-// than pow, which took 250 instructions a call (an eighth of the FP32
-// water_pass_a's).
+template <typename T>
 __device__ __forceinline__ double tait(double r, double gamma) {
-    if (gamma == 7.0) {
-        const double r2 = r * r, e2 = fma(r, r, -r2);
-        const double r3 = r2 * r, e3 = fma(r2, r, -r3) + e2 * r;
-        const double r6 = r3 * r3, e6 = fma(r3, r3, -r6) + 2.0 * r3 * e3;
-        const double r7 = r6 * r, e7 = fma(r6, r, -r7) + e6 * r;
-        return (r7 - 1.0) + e7;
-    }
-    return pow(r, gamma) - 1;
+    if (sizeof(T) == 8 || gamma != 7.0) return pow(r, gamma) - 1;
+    const double r2 = r * r, e2 = fma(r, r, -r2);
+    const double r3 = r2 * r, e3 = fma(r2, r, -r3) + e2 * r;
+    const double r6 = r3 * r3, e6 = fma(r3, r3, -r6) + 2.0 * r3 * e3;
+    const double r7 = r6 * r, e7 = fma(r6, r, -r7) + e6 * r;
+    return isinf(r7) ? r7 : (r7 - 1.0) + e7;
 }
 
 // What water_pass_a does with a particle's sums: EOS, newtonian_fluid, the
@@ -618,7 +621,7 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
         txx = c23 * (T(2) * t0 - t1);
         txy = t2 + t3;
         tyy = c23 * (T(2) * t1 - t0);
-        p = rho > 0.0 ? c.tab[sid].w_b * tait(rho / c.w_rho0, c.w_gamma) : pold;
+        p = rho > 0.0 ? c.tab[sid].w_b * tait<T>(rho / c.w_rho0, c.w_gamma) : pold;
         vof = 1.0;
     } else {
         drho = con + dl;
@@ -631,8 +634,8 @@ __device__ __forceinline__ void water_a_finish(const PhaseDev<T>& P, const SimCo
             if (c.volume_fraction) vof = half_step(vof, st.dt, fold);
         }
         const double ratio = rho / (c.w_rho0 * vof);
-        p = st.w_b * tait(ratio, c.w_gamma);
-        cnew = st.w_c * cube(ratio);
+        p = st.w_b * tait<T>(ratio, c.w_gamma);
+        cnew = st.w_c * cube<T>(ratio);
         P.c[a] = cnew;
     }
     P.drho[a] = drho;
