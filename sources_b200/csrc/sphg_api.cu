@@ -957,10 +957,15 @@ struct Engine : EngineBase {
     // FP32 with one h for all particles: two particles per lane pair in
     // packed FP32 arithmetic (sphg_pairs2.cuh); else one particle per lane.
     bool paired() const { return sizeof(T) == 4 && sc_same.uniform; }
-    // dspp: the wall force's r0
+    // dspp: the wall force's r0.  h: the soil passes take it as it is, since an
+    // error of a constant is common to all pairs of a sum (p of a column after six
+    // steps is 6 % to 26 % closer to FP64 than the one-particle passes', and with h
+    // rounded to FP32 first was up to 17 % further off).  The water passes take the
+    // rounded h, as the one-particle passes do: their sums were as close or closer
+    // (momentum 0.88 of those passes' error, XSPH 0.90 to 1.06, dvof 0.86).
     template <int SKF>
-    PairK pair_k(double dspp = 0.0) const {
-        const double h = (double)(float)hrange[0][1], pi = SPHG_PI_REF;
+    PairK pair_k(double h, double dspp = 0.0) const {
+        const double pi = SPHG_PI_REF;
         PairK K{};
         K.h = (float)h;
         K.nih = (float)(-1.0 / h);
@@ -971,7 +976,7 @@ struct Engine : EngineBase {
             K.ks = (float)(-fac / (2.0 * h)); K.kw = (float)(fac / 6.0);
         } else if (SKF == 4) {
             const double fac = 7.0 / (4.0 * pi * h * h);
-            K.ks = (float)(-5.0 * fac / (h * h)); K.kw = (float)fac;
+            K.ks = (float)(-0.625 * fac / (h * h)); K.kw = (float)(fac / 16.0);
         }
         const bool visc = sim.visc_artificial != 0;
         K.nh = (float)-h;
@@ -981,6 +986,7 @@ struct Engine : EngineBase {
         K.alpha_c = (float)(2.0 * sim.s_c);
         K.r0 = (float)dspp; K.dd = (float)(sim.dd / (double)K.ks); K.p1 = (float)sim.p1; K.p2 = (float)sim.p2;
         K.kb = (float)sim.s_kb;
+        K.dh = sim.delta * hrange[0][1];
         K.thr = sc_same.r2_uniform;
         return K;
     }
@@ -990,7 +996,7 @@ struct Engine : EngineBase {
         if constexpr (sizeof(T) == 4)
             if (paired())
                 return launch_pdl("water_pass_a", k_water_pass_a2<SKF>, blocks2(D.n), SPHG_TPB2, Staged2<false>::BYTES, D, grid,
-                                  pair_k<SKF>(), sim, cnt);
+                                  pair_k<SKF>((float)hrange[0][1]), sim, cnt);
         return with_lanes(D.n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             return launch_pdl("water_pass_a", k_water_pass_a<T, SKF, false, G>, blocksG(D.n, G), SPHG_TPB,
@@ -1030,7 +1036,7 @@ struct Engine : EngineBase {
         if constexpr (sizeof(T) == 4)
             if (paired())
                 return launch_pdl("water_pass_b", k_water_pass_b2<SKF, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O,
-                                  grid, pair_k<SKF>(D.dspp), sim, u, cnt);
+                                  grid, pair_k<SKF>((float)hrange[0][1], D.dspp), sim, u, cnt);
         return with_lanes(D.n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             return launch_pdl("water_pass_b", k_water_pass_b<T, SKF, false, FCH, G>, blocksG(D.n, G), SPHG_TPB, 0, D, O, grid,
@@ -1042,7 +1048,7 @@ struct Engine : EngineBase {
         if constexpr (sizeof(T) == 4)
             if (paired())
                 return launch_pdl("soil_pass", k_soil_pass2<SKF, SINGLE, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O, grid,
-                                  pair_k<SKF>(D.dspp), sim, cnt, slot, u);
+                                  pair_k<SKF>(hrange[0][1], D.dspp), sim, cnt, slot, u);
         return with_lanes(D.n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             return launch_pdl("soil_pass", k_soil_pass<T, SKF, SINGLE, FCH, G>, blocksG(D.n, G), SPHG_TPB, 0, D, O, grid, sc_same,

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_A2) k_water_pass_a2(Phase
     if (p.v0) P.hmask[p.k] = mask;   // a lane without a particle of its own still has its half of the pair's candidates
     if (p.valid) {
         // delta_sph: 2 delta h c (rho_a - rho_b), c of the previous EOS call
-        const float d = c.artificial_density ? -2.0f * K.ks * (float)(c.delta * (double)K.h * P.c[P.perm[p.k]]) * dl_ : 0.0f;
+        const float d = c.artificial_density ? -2.0f * K.ks * (float)(K.dh * P.c[P.perm[p.k]]) * dl_ : 0.0f;
         const float c23 = K.ks * (2.0f / 3.0f);
         water_a_finish<float, false>(P, c, p.k, -K.ks * con_, d, c23 * (2.0f * ta_ - tb_), K.ks * tc_, c23 * (2.0f * tb_ - ta_),
                                      0.0f, hits);
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_B2) k_water_pass_b2(Phase
     if (p.valid) {
         const RecB<float> q = P.recB[p.k];
         w.mx *= -K.ks * q.vof; w.my *= -K.ks * q.vof;
-        w.dvf *= c.water_artificial_volume ? -2.0f * K.ks * (float)(c.delta * (double)K.h) * q.c : 0.0f;
+        w.dvf *= c.water_artificial_volume ? -2.0f * K.ks * (float)K.dh * q.c : 0.0f;
         water_b_finish<float, false>(P, g, c, u, cnt, p.k, p.lane ? o.rho.y : o.rho.x, q.vof, w);
     }
     count_stats_redux(cnt, 2, -1, w.chits, p.valid);
@@ -309,8 +309,9 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_S2) k_soil_pass2(PhaseDev
             const float2 sxx = fma2(nfa, add2(nsx, neg2(npa)), splat2(fmaf(qb.sxx, fb, -pb)));
             const float2 syy = fma2(nfa, add2(nsy, neg2(npa)), splat2(fmaf(qb.syy, fb, -pb)));
             const float2 sxy = mul2(mw, fma2(nfa, nsxy, splat2(qb.sxy * fb)));
-            mx = fma2(sxy, gy, fma2(fma2(mw, sxx, pi), gx, mx));
-            my = fma2(sxy, gx, fma2(fma2(mw, syy, pi), gy, my));
+            // the pair's two parts first, so that the sum itself is rounded once a pair
+            mx = add2(fma2(sxy, gy, mul2(fma2(mw, sxx, pi), gx)), mx);
+            my = add2(fma2(sxy, gx, mul2(fma2(mw, syy, pi), gy)), my);
             if (!SINGLE && qb.itype < 0.0f) wall_pair(K, rr, dx, dy, h0 && real0, h1 && real1, mx, my);
         };
         visit_pairs<true>(P, g, p, &cnt->timeout, [&](const Runs3& r, const double2* xs, const RecA<float>* RA,
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_S2) k_soil_pass2(PhaseDev
     w.xsx = K.kw * p.mine(xx); w.xsy = K.kw * p.mine(xy);
     w.txx = c23 * (2.0f * ta_ - tb_); w.txy = K.ks * (tc_ + td_); w.tyy = c23 * (2.0f * tb_ - ta_);
     w.vcc = K.ks * (ta_ + tb_); w.wxy = 0.5f * K.ks * (tc_ - td_);
-    const float dh2 = -2.0f * K.ks * (float)(c.delta * (double)K.h);
+    const float dh2 = -2.0f * K.ks * (float)K.dh;
     const float ps = c.soil_artificial_stress ? dh2 * (float)c.s_c : 0.0f;
     w.dp = ps * p.mine(dpp); w.dsx = ps * p.mine(dsx); w.dsxy = ps * p.mine(dsxy); w.dsy = ps * p.mine(dsy);
     w.cdx = w.cdy = w.cpx = w.cpy = 0.0f;

@@ -50,6 +50,7 @@ struct PairK {
     float nh, h2e, alpha, beta, alpha_c;   // -h, etq^2 h^2, alpha/2 and beta of art_visc, alpha c_soil
     float r0, dd, p1, p2;     // wall force; dd over ks
     float kb;                 // Forchheimer
+    double dh;                // delta h of delta-SPH
     double thr;               // exact squared pair-test threshold
 };
 
@@ -59,17 +60,16 @@ template <int SKF>
 __device__ __forceinline__ void kernel_pair(const PairK& K, float2 r2, bool h0, bool h1, float2& w, float2& s) {
     if constexpr (SKF == 1 || SKF == 4) {
         const float2 rinv = make_float2(rsqrt_approx(fmaxf(r2.x, 1e-30f)), rsqrt_approx(fmaxf(r2.y, 1e-30f)));
-        const float2 nq = mul2(mul2(r2, rinv), splat2(K.nih));   // -q
+        const float2 r = mul2(r2, rinv), nq = mul2(r, splat2(K.nih));   // -q
+        const float2 u = fma2(r, splat2(K.nih), splat2(2.0f));   // 2 - q, rounded once: W and grad W are powers of it
         if constexpr (SKF == 1) {   // W = fac/6 (4 - 6 q^2 + 3 q^3 | (2-q)^3), s = -fac/(2h) ((4 - 3q)/h | (2-q)^2 / r)
             const float2 wn = fma2(mul2(nq, nq), fma2(splat2(-3.0f), nq, splat2(-6.0f)), splat2(4.0f));
             const float2 sn = fma2(splat2(K.sn1), nq, splat2(K.sn0));
-            const float2 u = add2(nq, splat2(2.0f));
             const float2 uu = mul2(u, u);
             const float2 wf = mul2(uu, u), sf = mul2(uu, rinv);
             w = sel2(h0, h1, make_float2(nq.x >= -1.0f ? wn.x : wf.x, nq.y >= -1.0f ? wn.y : wf.y));
             s = sel2(h0, h1, make_float2(nq.x >= -1.0f ? sn.x : sf.x, nq.y >= -1.0f ? sn.y : sf.y));
-        } else {   // the gradient polynomial -5 + 15q/2 - 15q^2/4 + 5q^3/8 is -5 (1 - q/2)^3
-            const float2 u = fma2(splat2(0.5f), nq, splat2(1.0f));
+        } else {   // the gradient polynomial -5 + 15q/2 - 15q^2/4 + 5q^3/8 is -5/8 (2 - q)^3
             const float2 uu = mul2(u, u);
             w = sel2(h0, h1, mul2(mul2(uu, uu), fma2(splat2(-2.0f), nq, splat2(1.0f))));
             s = sel2(h0, h1, mul2(uu, u));
