@@ -579,6 +579,10 @@ __global__ void __launch_bounds__(SPHG_TPB) k_water_sum(PhaseDev<T> P, GridGeom 
     count_stats(cnt, 0, 0, hits, finish);
 }
 
+// A particle's own density in the mean densities of the FP64 passes: an infinite
+// one as 1e200, whose reciprocal is zero for every purpose and has a residual.
+template <typename T> __device__ __forceinline__ T finite_rho(T rho) { return sizeof(T) == 8 && rho > T(1e200) ? T(1e200) : rho; }
+
 // The powers of the Tait equation, r^gamma - 1, and of the sound speed, r^3.  FP64
 // calls pow, as the reference does.  The single-precision mode (whose equation
 // of state is in FP64 all the same) takes gamma = 7, the exponent of water, and the cube
@@ -909,6 +913,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
     fa_a.x = fa_xx; fa_a.y = fa_xy; fa_b.x = fa_xy; fa_b.y = fa_yy;
     va.x = ra.vx; va.y = ra.vy;
     const uint4 mask = G == 1 && valid ? P.hmask[k] : make_uint4(0u, 0u, 0u, 0u);   // recorded by the step's first water pass
+    const T rho_m = finite_rho(ra.rho);
     auto body = [&](const RecA<T>* RA, const RecB<T>* RB, int m, T dx, T dy) {
         const RecA<T> rb = RA[m];
         const RecB<T> qb = RB[m];
@@ -932,7 +937,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_B : SPHG_
         // 1 / mean density (art_visc and av_vel); in FP64 from one division with 1 / (r^2 + etq^2 h^2), then corrected
         T irho, iden = T(0), den = T(0);
         if constexpr (sizeof(T) == 8) {
-            const T mr = T(0.5) * (ra.rho + rb.rho);
+            const T mr = T(0.5) * (rho_m + rb.rho);
             den = fmax(rr + mh * mh * etq2, T(1e-300));
             const T inv = T(1) / (mr * den);
             irho = rcp_near(mr, inv * den);
@@ -1143,6 +1148,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
     T s1x = 0, s1y = 0, s2x = 0, s3x = 0, s2y = 0, s3y = 0;
     T avx = 0, avy = 0, rpx = 0, rpy = 0, xsx = 0, xsy = 0;
     T dpp = 0, dsx = 0, dsxy = 0, dsy = 0;
+    const T rho_m = finite_rho(ra.rho);
     auto body = [&](int m, T dx, T dy) {
         const RecA<T> rb = P.recA[m];
         const RecB<T> qb = P.recB[m];
@@ -1154,7 +1160,7 @@ __global__ void __launch_bounds__(SPHG_TPB, sizeof(T) == 4 ? SPHG_MINB_SOIL : SP
         const T e = T(2) * sr;                            // 2 (dx . grad W) / r^2
         // in FP64, 1 / mean density, 1 / (r^2 + etq^2 h^2) and 1 / rho_b from one division (corrected where they are used)
         T irho64 = T(0), iden64 = T(0), irb64 = T(0), den = T(0);
-        const T mr = T(0.5) * (ra.rho + rb.rho);
+        const T mr = T(0.5) * (rho_m + rb.rho);
         if constexpr (sizeof(T) == 8) {
             den = fmax(rr + mh * mh * etq2, T(1e-300));
             const T md = mr * den, inv = T(1) / (md * rb.rho);
