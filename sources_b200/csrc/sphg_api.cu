@@ -957,12 +957,12 @@ struct Engine : EngineBase {
     // FP32 with one h for all particles: two particles per lane pair in
     // packed FP32 arithmetic (sphg_pairs2.cuh); else one particle per lane.
     bool paired() const { return sizeof(T) == 4 && sc_same.uniform; }
-    // dspp: the wall force's r0.  h: the soil passes take it as it is, since an
+    // dspp: the wall force's r0.  h: the soil-only pass takes it as it is, since an
     // error of a constant is common to all pairs of a sum (p of a column after six
-    // steps is 6 % to 26 % closer to FP64 than the one-particle passes', and with h
-    // rounded to FP32 first was up to 17 % further off).  The water passes take the
-    // rounded h, as the one-particle passes do: their sums were as close or closer
-    // (momentum 0.88 of those passes' error, XSPH 0.90 to 1.06, dvof 0.86).
+    // steps is 6 % to 26 % closer to FP64 than the one-particle pass's, and with h
+    // rounded to FP32 first was up to 17 % further off).  The two-phase passes take
+    // the rounded h, as the one-particle passes do: their sums were as close or
+    // closer (water: momentum 0.88 of those passes' error, XSPH 0.90 to 1.06).
     template <int SKF>
     PairK pair_k(double h, double dspp = 0.0) const {
         const double pi = SPHG_PI_REF;
@@ -1048,7 +1048,7 @@ struct Engine : EngineBase {
         if constexpr (sizeof(T) == 4)
             if (paired())
                 return launch_pdl("soil_pass", k_soil_pass2<SKF, SINGLE, FCH>, blocks2(D.n), SPHG_TPB2, Staged2<true>::BYTES, D, O, grid,
-                                  pair_k<SKF>(hrange[0][1], D.dspp), sim, cnt, slot, u);
+                                  pair_k<SKF>(SINGLE ? hrange[0][1] : (float)hrange[0][1], D.dspp), sim, cnt, slot, u);
         return with_lanes(D.n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             return launch_pdl("soil_pass", k_soil_pass<T, SKF, SINGLE, FCH, G>, blocksG(D.n, G), SPHG_TPB, 0, D, O, grid, sc_same,

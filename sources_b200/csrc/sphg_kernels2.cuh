@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_A2) k_water_pass_a2(Phase
                         [&](int m, float2 dx, float2 dy, bool h0, bool h1) {
             const RecA<float> rb = RA[m];
             float2 w, s;
-            kernel_pair<SKF>(K, fma2(dx, dx, mul2(dy, dy)), h0, h1, w, s);
+            kernel_pair<SKF, true>(K, fma2(dx, dx, mul2(dy, dy)), h0, h1, w, s);
             const float2 vs = mul2(splat2(rb.vol), s);
             const float2 gx = mul2(vs, dx), gy = mul2(vs, dy);   // vol_b grad W
             dl = fma2(vs, add2(splat2(rb.rho), nrho), dl);
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_B2) k_water_pass_b2(Phase
         auto body = [&](const RecA<float>& rb, const RecB<float>& qb, float2 dx, float2 dy, bool h0, bool h1) {
             const float2 rr = fma2(dx, dx, mul2(dy, dy));
             float2 w, s, mi, pi;
-            kernel_pair<SKF>(K, rr, h0, h1, w, s);
+            kernel_pair<SKF, false>(K, rr, h0, h1, w, s);
             const float2 gx = mul2(s, dx), gy = mul2(s, dy), vb = splat2(rb.vol);
             const float2 vp = mul2(vb, add2(pa, splat2(qb.p)));
             d1x = fma2(vp, gx, d1x);
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_B2) k_water_pass_b2(Phase
                 const RecA<float> rb = S.recA[m];
                 const float phis = S.recB[m].vof;
                 float2 w, s;
-                kernel_pair<SKF>(K, fma2(dx, dx, mul2(dy, dy)), h0, h1, w, s);
+                kernel_pair<SKF, false>(K, fma2(dx, dx, mul2(dy, dy)), h0, h1, w, s);
                 const float2 ux = add2(splat2(rb.vx), o.nu), uy = add2(splat2(rb.vy), o.nv);
                 float2 q = mul2(splat2(rb.vol * phis), w);
                 if constexpr (FCH) {
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_S2) k_soil_pass2(PhaseDev
         auto body = [&](const RecA<float>& rb, const RecB<float>& qb, float2 dx, float2 dy, bool h0, bool h1) {
             const float2 rr = fma2(dx, dx, mul2(dy, dy));
             float2 w, s, mi, pi;
-            kernel_pair<SKF>(K, rr, h0, h1, w, s);
+            kernel_pair<SKF, SINGLE>(K, rr, h0, h1, w, s);
             const float2 gx = mul2(s, dx), gy = mul2(s, dy);
             const float2 du = add2(splat2(rb.vx), o.nu), dv = add2(splat2(rb.vy), o.nv);   // v_b - v_a
             const float2 vb = splat2(rb.vol), vu = mul2(vb, du), vv = mul2(vb, dv);
@@ -309,9 +309,14 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_S2) k_soil_pass2(PhaseDev
             const float2 sxx = fma2(nfa, add2(nsx, neg2(npa)), splat2(fmaf(qb.sxx, fb, -pb)));
             const float2 syy = fma2(nfa, add2(nsy, neg2(npa)), splat2(fmaf(qb.syy, fb, -pb)));
             const float2 sxy = mul2(mw, fma2(nfa, nsxy, splat2(qb.sxy * fb)));
-            // the pair's two parts first, so that the sum itself is rounded once a pair
-            mx = add2(fma2(sxy, gy, mul2(fma2(mw, sxx, pi), gx)), mx);
-            my = add2(fma2(sxy, gx, mul2(fma2(mw, syy, pi), gy)), my);
+            const float2 cx = fma2(mw, sxx, pi), cy = fma2(mw, syy, pi);
+            if constexpr (SINGLE) {   // the pair's two parts first, so that the sum itself is rounded once a pair
+                mx = add2(fma2(sxy, gy, mul2(cx, gx)), mx);
+                my = add2(fma2(sxy, gx, mul2(cy, gy)), my);
+            } else {
+                mx = fma2(sxy, gy, fma2(cx, gx, mx));
+                my = fma2(sxy, gx, fma2(cy, gy, my));
+            }
             if (!SINGLE && qb.itype < 0.0f) wall_pair(K, rr, dx, dy, h0 && real0, h1 && real1, mx, my);
         };
         visit_pairs<true>(P, g, p, &cnt->timeout, [&](const Runs3& r, const double2* xs, const RecA<float>* RA,
@@ -337,7 +342,7 @@ __global__ void __launch_bounds__(SPHG_TPB2, SPHG_MINB_S2) k_soil_pass2(PhaseDev
                 const RecA<float> rb = W.recA[m];
                 const RecB<float> qb = W.recB[m];
                 float2 w, s;
-                kernel_pair<SKF>(K, fma2(dx, dx, mul2(dy, dy)), h0, h1, w, s);
+                kernel_pair<SKF, false>(K, fma2(dx, dx, mul2(dy, dy)), h0, h1, w, s);
                 float2 q = mul2(splat2(rb.vol * rb.rho * qb.vof), w);
                 const float2 ux = add2(splat2(rb.vx), o.nu), uy = add2(splat2(rb.vy), o.nv);
                 if constexpr (FCH) {

@@ -55,13 +55,17 @@ struct PairK {
 };
 
 // The shapes w' and s' of two pairs (W = kw w', grad W = ks s' dx); the halves
-// whose pair is no neighbour (hit false) get zero.
-template <int SKF>
+// whose pair is no neighbour (hit false) get zero.  FU: 2 - q, whose powers the
+// kernels are, in one multiply-add, so rounded once (water_pass_a and the
+// soil-only pass; the momentum and cross sums of the two-phase passes were as close
+// to FP64 with q rounded first, and keep that: a run held against the oracle there
+// has a particle within a rounding of yielding).
+template <int SKF, bool FU>
 __device__ __forceinline__ void kernel_pair(const PairK& K, float2 r2, bool h0, bool h1, float2& w, float2& s) {
     if constexpr (SKF == 1 || SKF == 4) {
         const float2 rinv = make_float2(rsqrt_approx(fmaxf(r2.x, 1e-30f)), rsqrt_approx(fmaxf(r2.y, 1e-30f)));
         const float2 r = mul2(r2, rinv), nq = mul2(r, splat2(K.nih));   // -q
-        const float2 u = fma2(r, splat2(K.nih), splat2(2.0f));   // 2 - q, rounded once: W and grad W are powers of it
+        const float2 u = FU ? fma2(r, splat2(K.nih), splat2(2.0f)) : add2(nq, splat2(2.0f));   // 2 - q
         if constexpr (SKF == 1) {   // W = fac/6 (4 - 6 q^2 + 3 q^3 | (2-q)^3), s = -fac/(2h) ((4 - 3q)/h | (2-q)^2 / r)
             const float2 wn = fma2(mul2(nq, nq), fma2(splat2(-3.0f), nq, splat2(-6.0f)), splat2(4.0f));
             const float2 sn = fma2(splat2(K.sn1), nq, splat2(K.sn0));
