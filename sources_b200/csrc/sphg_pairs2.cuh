@@ -7,7 +7,9 @@
 // BOTH particles for each candidate in Blackwell's packed FP32 arithmetic
 // (fma/mul/add.rn.f32x2), one particle in each half.  A candidate that is a
 // neighbour of only one of the two gets the kernel values W = 0 and grad W = 0
-// in the other half.  At the end the lanes swap halves (one shuffle per sum)
+// in the other half.  (0 times the infinity or NaN of a candidate is NaN, so a
+// particle whose sums come out not finite visits its own neighbours once more,
+// alone: visit_alone.)  At the end the lanes swap halves (one shuffle per sum)
 // and each finishes its own particle.  The pair test stays the exact FP64 one.
 //
 // Why: the passes are bound by instruction issue (129 and 143 warp
@@ -140,6 +142,8 @@ struct LanePair {
     __device__ __forceinline__ float mine(float2 v) const {
         return (lane ? v.y : v.x) + __shfl_xor_sync(0xffffffffu, lane ? v.x : v.y, 1);
     }
+    // this lane's particle's half alone
+    __device__ __forceinline__ float own(float2 v) const { return lane ? v.y : v.x; }
     __device__ __forceinline__ int mine(int h0, int h1) const {
         return (lane ? h1 : h0) + __shfl_xor_sync(0xffffffffu, lane ? h0 : h1, 1);
     }
@@ -265,6 +269,27 @@ __device__ __forceinline__ void pair_replay(const Runs3& r, int lane, double thr
              make_float2((float)(x0.y - xb.y), (float)(x1.y - xb.y)), (mask.x & bit) != 0u, (mask.z & bit) != 0u);
     }
 }
+
+// The lane's own particle's neighbours, and no other candidate, by the lane alone
+// (nothing of it is shared with other lanes): body as in pair_scan, with the
+// other half inactive and its sums left to be ignored.
+template <class F>
+__device__ __forceinline__ void visit_alone(const GridGeom& g, const int* __restrict__ cstart, double thr, const double2* xs,
+                                            const LanePair& p, int self, F&& body) {
+    const Runs3 r = row_runs(g, cstart, p.cx, p.cx, p.cy);
+    const double2 xa = p.lane ? p.x1 : p.x0;
+#pragma unroll 1
+    for (int t = 0; t < r.tot; ++t) {
+        const int m = r.at(t);
+        const double2 xb = xs[m];
+        const double dx = xa.x - xb.x, dy = xa.y - xb.y;
+        if (m != self && __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) < thr)
+            body(m, splat2((float)dx), splat2((float)dy), p.lane == 0, p.lane == 1);
+    }
+}
+__device__ __forceinline__ bool all_finite() { return true; }
+template <typename... R>
+__device__ __forceinline__ bool all_finite(float v, R... rest) { return isfinite(v) && all_finite(rest...); }
 
 // count_stats with the warp's integer reductions
 __device__ __forceinline__ void count_stats_redux(DevCounters* cnt, int list, int phase_slot, int hits, bool valid) {
