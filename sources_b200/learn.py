@@ -246,7 +246,6 @@ class MPNet:
         self.err = t.zeros(1, dtype=t.int32, device=self.device)
         self.loss_buf = t.zeros(1, dtype=t.float32, device=self.device)
         self.adam_step = 0
-        self.adam_list = None    # the tensors of sphg_gnn_adam_all, made at the first step
         # inputs include the displacement since the reference positions
         self.use_x0 = True
         # normalisation: velocity scale, acceleration mean (2) and std (2)
@@ -399,6 +398,9 @@ class MPNet:
     # ------------------------------------------------------------ backward
     def zero_grad(self):
         self.grads.zero_()
+        for d in list(self.W.values()) + list(self.B.values()):
+            if d["g"]._base is not self.grads:   # replaced by the program
+                d["g"].zero_()
 
     def loss(self, b: Batch, out, delta: float = 0.0):
         """Masked mean squared error over the 2 acceleration columns (Huber
@@ -490,12 +492,12 @@ class MPNet:
 
     def adam(self, lr: float, b1=0.9, b2=0.999, eps=1e-8):
         self.adam_step += 1
-        if self.adam_list is None:
-            ts = list(self.W.values()) + list(self.B.values())
-            self.adam_list = AdamList(len(ts), 0, (AdamTensor * ADAM_MAX)(*[
-                AdamTensor(*(_ptr(d.get(k)) for k in ("w", "g", "m", "v", "wb", "wt")), d["rows"], d.get("cols", 1),
-                           d["lim"], 0) for d in ts]))
-        self._k("sphg_gnn_adam_all", C.addressof(self.adam_list), lr, b1, b2, eps, self.adam_step, self.stream)
+        # from the tensors as they are now: a program may have replaced one since the last step
+        ts = list(self.W.values()) + list(self.B.values())
+        lst = AdamList(len(ts), 0, (AdamTensor * ADAM_MAX)(*[
+            AdamTensor(*(_ptr(d.get(k)) for k in ("w", "g", "m", "v", "wb", "wt")), d["rows"], d.get("cols", 1), d["lim"], 0)
+            for d in ts]))
+        self._k("sphg_gnn_adam_all", C.addressof(lst), lr, b1, b2, eps, self.adam_step, self.stream)
 
     def check_device_errors(self):
         if int(self.err.item()) != 0:
