@@ -169,6 +169,10 @@ struct PinnedCopies {
     // 0 done (upwards: the host arrays are no longer read), 1 error, -1 not taken (page-locked arrays only, a
     // device address among them, or no buffer)
     int run(const std::vector<Seg>& s, char* dev, size_t total, bool up, cudaStream_t st, int device) {
+        // cudaStreamPerThread is another stream in each thread: the calling thread then works alone, and uploads,
+        // which one thread moves no faster than the driver, stay with the driver
+        const bool shared = st != cudaStreamPerThread;
+        if (total == 0 || (up && (total < kUpBytes || !shared))) return -1;
         bool any = false;
         for (const Seg& g : s) {
             for (const char* h : {g.h0, g.h1}) {
@@ -177,10 +181,7 @@ struct PinnedCopies {
                 any = any || t == cudaMemoryTypeUnregistered;
             }
         }
-        // cudaStreamPerThread is another stream in each thread: the calling thread then works alone, and uploads,
-        // which one thread moves no faster than the driver, stay with the driver
-        const bool shared = st != cudaStreamPerThread;
-        if (!any || total == 0 || (up && (total < kUpBytes || !shared))) return -1;
+        if (!any) return -1;
         Slot* slot[kWorkers];
         int nw = 0;
         for (const int want = total >= kThreadBytes && shared ? kWorkers : 1; nw < want; ++nw)
