@@ -1000,7 +1000,7 @@ struct Engine : EngineBase {
         return with_lanes(D.n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             return launch_pdl("water_pass_a", k_water_pass_a<T, SKF, false, G>, blocksG(D.n, G), SPHG_TPB,
-                              G == 1 ? (size_t)SPHG_STAGE_A * (16 + sizeof(RecA<T>)) : 0, D, grid, sc_same, sim, cnt);
+                              G == 1 && sc_same.uniform ? (size_t)SPHG_STAGE_A * (16 + sizeof(RecA<T>)) : 0, D, grid, sc_same, sim, cnt);
         });
     }
     // FP64 phases too small to fill the GPU: 8 or 4 lanes per particle
