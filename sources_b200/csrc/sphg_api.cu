@@ -1005,10 +1005,11 @@ struct Engine : EngineBase {
     }
     // FP64 phases too small to fill the GPU: 8 or 4 lanes per particle
     // (scan_lanes), since one lane's walk of its candidates is all the time a
-    // pass takes there.  us per step with 1, 4, 8 and 16 lanes, water only: 4.6k
-    // particles 62.5, 43.2, 36.4, 36.5; 8.8k 66.0, 43.0, 39.0, 48.4; 17k 68.4,
-    // 47.2, 54.1; 34k 72.7, 66.2, 79.5; 50k 75.5, 86.5.  Soil only: 4.7k 46.6,
-    // 30.6, 28.1, 34.2; 9k 47.0, 32.3, 36.3; 34k 52.9, 54.9.
+    // pass takes there.  us per step with 1, 4 and 8 lanes, water only: 3.3k
+    // particles 56.9, 36.4, 30.3; 6.0k 59.2, 36.8, 32.5; 11k 59.6, 40.4, 41.8; 22k
+    // 65.3, 51.4, 60.4; 33k 68.7, 62.8, 75.6.  Soil only: 3.3k 42.4, 26.3, 23.7; 11k
+    // 44.5, 28.3, 32.5; 22k 46.6, 39.8, 45.0; 33k 48.7, 48.1, 55.0.  (16 lanes were no
+    // faster than 8 at 4.6k.)
     static int lanes(int n) { return sizeof(T) == 4 || n > 32000 ? 1 : n > 10000 ? 4 : 8; }
     template <class F>
     static int with_lanes(int n, F&& f) {   // f(integral_constant G)

@@ -1,18 +1,19 @@
 // sphg_kernels.cuh — the sm_100a kernels of libsphg.
 //
 // Per step (two-phase, declarations_sph.f90:525-791 with single_step :1131):
-//   k_first_half      leapfrog predictor (+ Drucker-Prager on soil)      elementwise
 //   k_cell_count      cell key per particle, rank inside its cell         elementwise
 //   k_cell_scatter    counting-sort scatter into cell order              elementwise
 //   k_cell_sort       order each cell by original index (reorder steps; else in the gather)  per cell
-//   k_gather          sorted copies: x, h, (v, m, rho); soil: DP + stress pair pass inputs
+//   k_gather          sorted copies: x, h, (v, m, rho) at the half step (the leapfrog predictor);
+//                     soil: DP + stress pair pass inputs
 //   k_water_sum       summation density (water-only step)                pair pass
 //   k_water_pass_a    continuity / df2, delta-SPH(rho), strain rate, EOS  pair pass
 //   k_water_pass_b    momentum, art. viscosity, delta-SPH(vof), wall force, XSPH  pair pass
 //   k_soil_pass       every same-phase soil term + flow rule + Jaumann   pair pass
 //   cross_soil_sums   Darcy drag + pore pressure on soil (in k_soil_pass) pair sums
 //   cross_water_sums  Darcy drag, dvof, vof2 on water (in k_water_pass_b) pair sums
-//   k_update          leapfrog corrector / first step (+ DP on soil)     elementwise
+//   Corrector         leapfrog corrector / first step (+ DP on soil), in the last pass of each phase
+// The FP32 passes of a step with soil and one h are in sphg_kernels2.cuh.
 // Every pair pass is a gather: one thread per particle in cell order visits
 // the 3 x 3 neighbouring cells (three contiguous row segments of the sorted
 // list), evaluates the reference's pair test bit-exactly in FP64 and sums the
@@ -47,7 +48,8 @@ struct SimConst {
 #define SPHG_X_SPLIT 4
 #endif
 // minimum resident blocks per SM of each pair pass (register cap for the
-// compiler: 65,536 / (SPHG_TPB * min blocks) registers per thread).  Timed on a B200 at 912,016 particles:
+// compiler: 65,536 / (SPHG_TPB * min blocks) registers per thread).  FP32: timed on a B200 at 912,016
+// particles of one h, before those ran the paired passes; now for the water-only step and several h.
 // water_pass_a (staged, recording the hit masks) 131 us at 8 blocks, 134 at
 // 7, 138 at 10 (48 registers).  water_pass_b (replaying the masks, with the
 // cross pairs) 176 us at 6 blocks, 164 at 7, 181 at 8 (spills).  soil_pass
@@ -58,11 +60,11 @@ struct SimConst {
 #ifndef SPHG_MINB_B
 #define SPHG_MINB_B 7
 #endif
-// neighbours of one block of the two-phase water_pass_a staged in shared
+// neighbours of one block of the two-phase water_pass_a (FP64 with one h) staged in shared
 // memory (records; the sizes of 128 consecutive particles' candidate runs at
 // dx = 0.002 m: mean 414, largest 544).  Each lane tests its candidates
 // from there one at a time and runs the pair body on each hit at once
-// (scan_direct): 123.5 us per launch at 912,016 particles, against 130.7 us
+// (scan_direct): in FP32, which runs it paired now, 123.5 us per launch at 912,016 particles, against 130.7 us
 // with the hit buffer that batches the bodies across the warp, and 130.4 us
 // for the direct scan reading through L1.
 #ifndef SPHG_STAGE_A
@@ -73,9 +75,10 @@ struct SimConst {
 #endif
 
 // FP64, 912,016 particles: serial chains of FP64 operations, hidden by resident
-// blocks.  water_pass_a 164 us at 4, 5 or 6; water_pass_b 317 uncapped (164
-// registers), 272 at 4, 474 at 5 (spills); soil_pass 139 uncapped (212), 109 at
-// 3, 140 at 4 (spills).
+// blocks.  water_pass_a 181 us uncapped, 184 at 5; water_pass_b 314 uncapped (166
+// registers), 273 at 4; soil_pass 140 uncapped (214), 112 at 3.  One block more of
+// either of the last two spills: 474 at 5 and 140 at 4, before the quotients'
+// corrections.
 #ifndef SPHG_MINB_A64
 #define SPHG_MINB_A64 5
 #endif

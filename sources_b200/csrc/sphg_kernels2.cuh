@@ -16,8 +16,9 @@
 //   soil_pass      86.7 ->  62.6 us   (5, 6, 8 blocks of 64: 64, 63, 63)
 //   step          421.3 -> 372.5 us
 // and with the epilogue's loads before its stores, no predictor stored and the
-// shorter cell list 85, 139, 58 and 314 us (issue slots 59, 49 and 40 % used,
-// 69, 97 and 177 warp instructions a particle);
+// shorter cell list 85, 139, 57 and 312 us; with the checks of the sums (below)
+// 86.5, 139.6, 57 and 314 (issue slots 58, 49 and 40 % used, 70, 98 and 177 warp
+// instructions a particle);
 // at 150k particles (Wendland, quadratic drag): 31.0 -> 27.1, 42.3 ->
 // 41.9, 43.5 -> 36.0 us; soil only, 190k: 67.6 -> 53.8 us.  Neighbours come
 // from shared memory: read through L1 (two particles and all candidates per
